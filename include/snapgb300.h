@@ -334,6 +334,20 @@ int sg_spmm_masked(int dtype, int block, int64_t rows, const int64_t* ptr, const
                    const void* in, void* out, const void* scale, const void* dshift, const void* y, int grid,
                    int variant, const unsigned char* row_mask, void* stream);
 
+/* FP64 SpMM of implicit-ones rows (sg_spmm with dtype 1, val = NULL) by     */
+/* exact fixed-point sums: each column of `in` (in_rows x block) is scaled by */
+/* a power of two, rounded once to 64-bit integers (error <= 2^-62 of the    */
+/* column's largest magnitude) and summed in 96 bits, so the sums do not     */
+/* depend on their order.  A non-finite value in `in` sends the call through */
+/* FP64 additions.  work: sg_spmm_fx_work_bytes(block, in_rows) bytes of     */
+/* device scratch, one per concurrent call; in / out / y / work 16-byte      */
+/* aligned.  No reference counterpart (an arithmetic form of the FP64        */
+/* matvec of embedding.rs:155-188).                                          */
+int64_t sg_spmm_fx_work_bytes(int block, int64_t in_rows);
+int sg_spmm_fx(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_rows, const double* in,
+               double* out, const double* scale, const double* dshift, const double* y, void* work,
+               int64_t work_bytes, void* stream);
+
 /* IDF weights from per-column cell counts (FP64, e.g. sg_col_counts of the */
 /* index pattern) with the rules of idf (embedding.rs:269-286): all counts   */
 /* equal -> 1, count 0 -> 1, count n -> n - 1, w = ln(n / count).  mm: two   */
@@ -517,8 +531,9 @@ typedef struct sg_lanczos_opts {
                             /* compensated FP32 kernels (sg_spmm_ds), 2 with */
                             /* FP64 kernels, 0 none                          */
   int variant_t, variant_x; /* SpMM kernel per pass (codes: < 100 gather,    */
-                            /* 100 + v stage-tiled, 200 + v dynamic); -1:    */
-                            /* library default                               */
+                            /* 100 + v stage-tiled, 200 + v dynamic, 300     */
+                            /* fixed point: FP64 without values, else as 1); */
+                            /* -1: library default                           */
   int refine_variant_t, refine_variant_x; /* SpMM of the sweep: refine 1,  */
                             /* sg_spmm_ds variants 0-3; refine 2, FP64      */
                             /* block-32 gather or dynamic codes; -1 default  */

@@ -49,19 +49,16 @@ def eigsum_grad(op: _eigen.GramOperator, evals: np.ndarray, U: torch.Tensor) -> 
     chk = _lib.check
     chk(L.sg_adjoint_stage1(n, k, U.data_ptr(), lam.data_ptr(), op.dinv.data_ptr(), op.rinv.data_ptr(), B1,
                             in1.data_ptr(), dbar.data_ptr(), sh), "adjoint stage 1")
-    chk(L.sg_spmm(1, B1, m, op.colptr.data_ptr(), op.rowidx.data_ptr(), cv.data_ptr() if cv is not None else None,
-                  in1.data_ptr(), zeh.data_ptr(), ones_m.data_ptr(), None, None, -1, sh), "adjoint Xᵀ pass")
+    _eigen.spmm64(m, op.colptr, op.rowidx, cv, n, in1, zeh, ones_m, B1, sh)                    # Xᵀ pass
     chk(L.sg_adjoint_stage2(m, k, zeh.data_ptr(), B1, op.w.data_ptr(), B2, in2.data_ptr(), sh), "adjoint stage 2")
-    chk(L.sg_spmm(1, B2, n, op.csr.indptr.data_ptr(), op.csr.indices.data_ptr(), v.data_ptr() if v is not None else None,
-                  in2.data_ptr(), P.data_ptr(), ones_n.data_ptr(), None, None, -1, sh), "adjoint X pass")
+    _eigen.spmm64(n, op.csr.indptr, op.csr.indices, v, m, in2, P, ones_n, B2, sh)              # X pass
     chk(L.sg_adjoint_stage3(n, k, U.data_ptr(), op.dinv.data_ptr(), op.rinv.data_ptr(), dbar.data_ptr(),
                             P.data_ptr(), B2, in3.data_ptr(), sh), "adjoint stage 3")
     cv2 = None
     if cv is not None:
         cv2 = torch.empty_like(cv)
         chk(L.sg_square_values(cv.numel(), cv.data_ptr(), cv2.data_ptr(), sh), "square values")
-    chk(L.sg_spmm(1, 4, m, op.colptr.data_ptr(), op.rowidx.data_ptr(), cv2.data_ptr() if cv2 is not None else None,
-                  in3.data_ptr(), g.data_ptr(), ones_m.data_ptr(), None, None, -1, sh), "adjoint (X∘X)ᵀ pass")
+    _eigen.spmm64(m, op.colptr, op.rowidx, cv2, n, in3, g, ones_m, 4, sh)                      # (X∘X)ᵀ pass
     chk(L.sg_adjoint_final(m, k, op.w.data_ptr(), zeh.data_ptr(), B1, g.data_ptr(), grad.data_ptr(), sh),
         "adjoint final")
     return grad

@@ -77,12 +77,6 @@ def rescale_chunks(q: torch.Tensor, evals: torch.Tensor, chunk_size: int) -> Non
         raise
 
 
-def _spmm64(rows, ptr, idx, val, inp, out, scale, block, stream):
-    L = _lib.load()
-    _lib.check(L.sg_spmm(1, block, rows, ptr.data_ptr(), idx.data_ptr(), None if val is None else val.data_ptr(),
-                         inp.data_ptr(), out.data_ptr(), scale.data_ptr(), None, None, -1, stream), "sg_spmm (FP64)")
-
-
 def orthogonalize(evals: np.ndarray, q: torch.Tensor):
     """``orthogonalize`` (``_embedding.py:397-413``): the eigenpairs of
     diag(σ) Vᵀ diag(λ) V diag(σ) from the SVD q = U diag(σ) Vᵀ, mapped back
@@ -194,10 +188,10 @@ def spectral_nystrom(X, features=None, n_comps: int = 30, sample_size: int = 100
             inp = torch.zeros(op_s.n, blk, **f64)
             inp[:, :kc] = ev[:, c0:c0 + kc] * op_s.rinv.unsqueeze(1)
             W = torch.empty(m, blk, **f64)
-            _spmm64(m, op_s.colptr, op_s.rowidx, op_s.cvalues, inp, W, w, blk, sh)
+            _eigen.spmm64(m, op_s.colptr, op_s.rowidx, op_s.cvalues, op_s.n, inp, W, w, blk, sh)
             W *= w.unsqueeze(1)
             Q = torch.empty(n, blk, **f64)
-            _spmm64(n, csr.indptr, csr.indices, csr.data, W, Q, rinv, blk, sh)
+            _eigen.spmm64(n, csr.indptr, csr.indices, csr.data, m, W, Q, rinv, blk, sh)
             q[:, c0:c0 + kc] = Q[:, :kc]
         rescale_chunks(q, torch.from_numpy(v).to(dev), chunk_size)
         evals, evecs = orthogonalize(v, q)

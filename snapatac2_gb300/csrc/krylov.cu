@@ -27,6 +27,7 @@ namespace {
 
 constexpr int kStaged = 100;
 constexpr int kDyn = 200;
+constexpr int kFx = 300;  // FP64 fixed-point sums (implicit ones)
 constexpr double kFp32Floor = 3e-5;  // residual level (x |A|) of a stalled FP32 solve
 
 // ---------------------------------------------------------------------------
@@ -262,6 +263,8 @@ struct Work {
   double *part, *C1, *C2, *G, *R1, *R2, *Rinv, *Rout, *H, *ctl, *theta_keep, *Yk, *Bc, *Yf, *evals_f, *res_f;
   int *ord, *sel, *row_of;
   unsigned* counter;
+  char* fx;  // scratch of the fixed-point SpMM (FP64 form)
+  int64_t fx_bytes;
   RitzLayout ritz;
   // correction sweep
   double *Up, *Zs64, *W64, *T64, *part32, *G32, *H32, *Ri, *Cs, *tmp, *Yr, *ev32;
@@ -283,6 +286,8 @@ Work layout(char* base, int code, int b, int k, int64_t n, int64_t m, int M, int
                 oYk = take((int64_t)ld * ld * 8), oBc = take((int64_t)b * ld * 8), oYf = take((int64_t)ld * k * 8),
                 oef = take((int64_t)k * 8), orf = take((int64_t)k * 8), ocnt = take(2 * 4),
                 oord = take((int64_t)ld * 4), osel = take((int64_t)ld * 4), orow = take((int64_t)ld * 4);
+  const int64_t fx_bytes = code ? sg_spmm_fx_work_bytes(b, std::max(n, m)) : 0;
+  const int64_t ofx = take(fx_bytes);
   const RitzLayout rl = ritz_layout(nullptr, M, M);
   const int64_t orl = take(rl.bytes);
   const bool refine = code == 0 && k <= 32;
@@ -307,6 +312,8 @@ Work layout(char* base, int code, int b, int k, int64_t n, int64_t m, int M, int
   w.ctl = (double*)(base + octl); w.theta_keep = (double*)(base + oth); w.Yk = (double*)(base + oYk);
   w.Bc = (double*)(base + oBc); w.Yf = (double*)(base + oYf); w.evals_f = (double*)(base + oef);
   w.res_f = (double*)(base + orf); w.counter = (unsigned*)(base + ocnt);
+  w.fx = fx_bytes ? base + ofx : nullptr;
+  w.fx_bytes = fx_bytes;
   w.ord = (int*)(base + oord); w.sel = (int*)(base + osel); w.row_of = (int*)(base + orow);
   w.ritz = ritz_layout(base + orl, M, M);
   if (refine) {
@@ -321,7 +328,7 @@ Work layout(char* base, int code, int b, int k, int64_t n, int64_t m, int M, int
 
 int default_variant(int code, int which) {
   if (code == 0) return which == 0 ? kDyn + 7 : 6;  // measured best at 100k x 500k, block 8
-  return 1;
+  return kFx;
 }
 
 // One operator application W = A Z (Zs = a ⊙ Z precomputed, T: m x B scratch)
@@ -331,6 +338,8 @@ struct Apply {
   cudaStream_t s;
   int* status;
   unsigned* counter;
+  char* fx;
+  int64_t fx_bytes;
   bool timed;
   std::vector<cudaEvent_t> ev;
   int64_t launches = 0, spmm_launches = 0;
@@ -344,6 +353,15 @@ struct Apply {
     const void* scale = code ? (const void*)(t ? op->w2 : op->a) : (const void*)(t ? op->w2_f32 : op->a_f32);
     const void* dsh = t ? nullptr : (code ? (const void*)op->dinv : (const void*)op->dinv_f32);
     const void* yy = t ? nullptr : y;
+    if (variant >= kFx) {
+      if (code && !val && fx) {
+        launches += 3;
+        ++spmm_launches;
+        return sg_spmm_fx(B, rows, ptr, idx, t ? op->n : op->m, (const double*)in, (double*)out, (const double*)scale,
+                          (const double*)dsh, (const double*)yy, fx, fx_bytes, s);
+      }
+      variant = 1;
+    }
     if (variant >= kDyn && code != 0) variant -= kDyn;  // the dynamic schedule is FP32 only
     int e;
     if (variant >= kDyn && t && op->order_t && op->order_t_positions > 0) {
@@ -472,7 +490,7 @@ extern "C" int sg_lanczos(const sg_gram_op* op, int precision, int block, int k,
   if (work_bytes < w.bytes) return SG_ERR_CAP;
   cudaStream_t s = as_stream(stream);
   const void* a = code ? (const void*)op->a : (const void*)op->a_f32;
-  Apply ap{op, s, status, w.counter, o.time_spmm != 0, {}};
+  Apply ap{op, s, status, w.counter, w.fx, w.fx_bytes, o.time_spmm != 0, {}};
   int64_t& nl = ap.launches;
   double ph_cycles = 0.0, ph_ritz = 0.0, ph_restart = 0.0, ph_refine = 0.0;
 #define SG_TRY(x)              \
