@@ -78,9 +78,13 @@ const char* sg_status_string(int status);
 /* Three calls:                                                              */
 /*  1. sg_tile_plan  -> key_ptr[n_cells+1]: exclusive prefix of the number   */
 /*     of tile hits ("keys") per cell; key_ptr[n_cells] = total keys K.      */
-/*  2. sg_tile_run   -> sorts and run-length-encodes each cell's keys into   */
-/*     scratch (sg_tile_scratch_bytes(K) bytes) and writes out_indptr        */
-/*     [n_cells+1]; out_indptr[n_cells] = nnz.                               */
+/*     Or, without reading a fragment and for every strategy but             */
+/*     SG_COUNT_FRAGMENT, sg_tile_bound -> an upper bound: two keys per      */
+/*     fragment (SG_COUNT_SINGLE: one), so K = 2 F (F); 2 F < 2^31.          */
+/*  2. sg_tile_run   -> counts each cell's keys into scratch                 */
+/*     (sg_tile_scratch_bytes(K) bytes) and writes out_indptr [n_cells+1];   */
+/*     out_indptr[n_cells] = nnz.  Both this call and the plan report a      */
+/*     fragment out of range (status, lowest index in *bad).                 */
 /*  3. sg_tile_emit  -> copies the (tile, count) pairs into out_idx/out_cnt  */
 /*     (capacity cap >= nnz).                                                */
 /* The result equals the reference's CSR: per row, tile indices strictly     */
@@ -91,6 +95,8 @@ int sg_tile_plan(const int64_t* cell_ptr, int64_t n_cells, int64_t n_frags, cons
                  const uint8_t* chrom_excl, int n_chrom, uint32_t bin_size, int strategy,
                  int64_t min_len, int64_t max_len, int64_t* key_ptr, void* scan_scratch,
                  int* status, unsigned long long* bad, void* stream);
+
+int sg_tile_bound(const int64_t* cell_ptr, int64_t n_cells, int strategy, int64_t* key_ptr, void* stream);
 
 /* Bytes of scratch needed by sg_tile_plan's scan (n_cells + 1 entries). */
 int64_t sg_scan_scratch_bytes(int64_t n);

@@ -40,6 +40,7 @@ SIGNATURES: dict[str, tuple] = {
     "sg_status_string": (ctypes.c_char_p, [_I32]),
     "sg_scan_scratch_bytes": (_I64, [_I64]),
     "sg_tile_scratch_bytes": (_I64, [_I64]),
+    "sg_tile_bound": (_I32, [_P, _I64, _I32, _P, _P]),
     "sg_tile_plan": (_I32, [_P, _I64, _I64, _P, _P, _P, _P, _P, _I32, _U32, _I32, _I64, _I64, _P, _P,
                             _P, _P, _P]),
     "sg_tile_run": (_I32, [_P, _I64, _I64, _P, _P, _P, _P, _P, _I32, _U32, _I32, _I64, _I64, _P, _P,
@@ -155,7 +156,7 @@ class LanczosInfo(ctypes.Structure):
 # benchmark): e.g. sg_block_cholqr = projection partial + reduce + Cholesky +
 # R⁻¹ application.
 KERNELS_PER_CALL = {
-    "sg_tile_plan": 4, "sg_tile_run": 5, "sg_tile_emit": 1, "sg_col_counts": 2, "sg_csr_select_cols": 5,
+    "sg_tile_plan": 4, "sg_tile_bound": 1, "sg_tile_run": 5, "sg_tile_emit": 1, "sg_col_counts": 2, "sg_csr_select_cols": 5,
     "sg_csr_transpose": 8, "sg_spectral_prepare": 7, "sg_spmm": 1, "sg_spmm_ex": 1, "sg_spmm_masked": 1, "sg_spmm_fx": 3,
     "sg_spmm_staged": 1, "sg_spmm_dyn": 1, "sg_spmm_ds": 1, "sg_ds_split": 1, "sg_spmm_dyn_ordered": 1, "sg_row_order": 10, "sg_idf_from_counts": 3, "sg_csr_row_norms": 1, "sg_staged_table": 1, "sg_gather_ceiling": 1, "sg_block_proj": 2, "sg_block_update": 1, "sg_block_cholqr": 4, "sg_block_finish": 1,
     "sg_lanczos_hblock": 1, "sg_basis_rotate": 1, "sg_fill_random": 1, "sg_knn": 6, "sg_knn_noalloc": 6,
@@ -231,9 +232,12 @@ def ptr(t: torch.Tensor | None) -> int | None:
 class DeviceStatus:
     """Device-side status word + lowest offending index (see the C header)."""
 
-    def __init__(self, device):
-        self.buf = torch.zeros(2, dtype=torch.int64, device=device)
-        self.buf[1] = -1  # 0xffff... as uint64: no offending entry yet
+    def __init__(self, device, buf: torch.Tensor | None = None):
+        """``buf``: two int64 of a larger device buffer to keep the words in,
+        so that one copy reads them together with their neighbours."""
+        self.buf = torch.empty(2, dtype=torch.int64, device=device) if buf is None else buf
+        self.buf[:1].zero_()
+        self.buf[1:].fill_(-1)  # 0xffff... as uint64: no offending entry yet
 
     @property
     def status_ptr(self) -> int:
@@ -244,7 +248,11 @@ class DeviceStatus:
         return self.buf.data_ptr() + 8
 
     def raise_if_error(self, what: str, index_name: str = "entry") -> None:
-        v = self.buf.cpu().tolist()
+        self.raise_if(self.buf.cpu().tolist(), what, index_name)
+
+    @staticmethod
+    def raise_if(v, what: str, index_name: str = "entry") -> None:
+        """Raise unless the two words ``v``, read back, say SG_OK."""
         st = int(v[0]) & 0xFFFFFFFF
         if st != SG_OK:
             bad = v[1] & 0xFFFFFFFFFFFFFFFF
