@@ -152,6 +152,34 @@ int sg_region_run(const int64_t* cell_ptr, int64_t n_cells, int64_t n_frags, con
                   int64_t min_len, int64_t max_len, const int64_t* key_ptr, void* scratch, int64_t scratch_bytes,
                   int64_t* out_indptr, void* scan_scratch, int* status, unsigned long long* bad, void* stream);
 
+/* Bucket index of the regions (n_regions = region_ptr[n_chrom]): for every  */
+/* 2^shift-th base of the genome (`genome` bases in all) the first region    */
+/* that starts there or later.  index: sg_region_index_bytes, 8-byte aligned. */
+int sg_region_index_shift(uint64_t genome, int64_t n_regions);
+int64_t sg_region_index_bytes(uint64_t genome, int64_t n_regions);
+int sg_region_index(uint64_t genome, const uint64_t* chrom_end, int n_chrom, const int64_t* region_ptr,
+                    const uint64_t* region_start, int64_t n_regions, void* index, int64_t index_bytes, void* stream);
+
+/* sg_region_plan / sg_region_run with the index (NULL: none) and a mask of  */
+/* (n_frags + 31) / 32 words (NULL: none) in which the plan marks the        */
+/* fragments that hit a region, the only ones that the run looks up again.   */
+/* Same results.                                                             */
+int sg_region_plan_indexed(const int64_t* cell_ptr, int64_t n_cells, int64_t n_frags, const uint64_t* frag_pos,
+                           const uint32_t* frag_len, const uint64_t* chrom_end, const uint8_t* chrom_excl,
+                           int n_chrom, const int64_t* region_ptr, const uint64_t* region_start,
+                           const uint64_t* region_end, const uint64_t* region_maxend, const uint32_t* region_id,
+                           int64_t n_features, int strategy, int64_t min_len, int64_t max_len, const void* index,
+                           uint64_t genome, int64_t n_regions, uint32_t* frag_mask, int64_t* key_ptr,
+                           void* scan_scratch, int* status, unsigned long long* bad, void* stream);
+int sg_region_run_indexed(const int64_t* cell_ptr, int64_t n_cells, int64_t n_frags, const uint64_t* frag_pos,
+                          const uint32_t* frag_len, const uint64_t* chrom_end, const uint8_t* chrom_excl,
+                          int n_chrom, const int64_t* region_ptr, const uint64_t* region_start,
+                          const uint64_t* region_end, const uint64_t* region_maxend, const uint32_t* region_id,
+                          int64_t n_features, int strategy, int64_t min_len, int64_t max_len, const void* index,
+                          uint64_t genome, int64_t n_regions, const uint32_t* frag_mask, const int64_t* key_ptr,
+                          void* scratch, int64_t scratch_bytes, int64_t* out_indptr, void* scan_scratch, int* status,
+                          unsigned long long* bad, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Fragment-file import -- replaces the PyO3 import_fragments               */
 /*   (snapatac2-python/src/preprocessing.rs:87-184) and                     */

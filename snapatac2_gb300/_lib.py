@@ -47,6 +47,13 @@ SIGNATURES: dict[str, tuple] = {
                            _I64, _P, _P, _P, _P, _P]),
     "sg_tile_emit": (_I32, [_I64, _P, _P, _I64, _P, _P, _P, _I64, _P, _P]),
     "sg_col_counts": (_I32, [_I64, _I64, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "sg_region_index_shift": (_I32, [ctypes.c_uint64, _I64]),
+    "sg_region_index_bytes": (_I64, [ctypes.c_uint64, _I64]),
+    "sg_region_index": (_I32, [ctypes.c_uint64, _P, _I32, _P, _P, _I64, _P, _I64, _P]),
+    "sg_region_plan_indexed": (_I32, [_P, _I64, _I64, _P, _P, _P, _P, _I32, _P, _P, _P, _P, _P, _I64, _I32, _I64, _I64,
+                                      _P, ctypes.c_uint64, _I64, _P, _P, _P, _P, _P, _P]),
+    "sg_region_run_indexed": (_I32, [_P, _I64, _I64, _P, _P, _P, _P, _I32, _P, _P, _P, _P, _P, _I64, _I32, _I64, _I64,
+                                     _P, ctypes.c_uint64, _I64, _P, _P, _P, _I64, _P, _P, _P, _P, _P]),
     "sg_region_plan": (_I32, [_P, _I64, _I64, _P, _P, _P, _P, _I32, _P, _P, _P, _P, _P, _I64, _I32, _I64, _I64,
                               _P, _P, _P, _P, _P]),
     "sg_region_run": (_I32, [_P, _I64, _I64, _P, _P, _P, _P, _I32, _P, _P, _P, _P, _P, _I64, _I32, _I64, _I64,
@@ -164,7 +171,7 @@ KERNELS_PER_CALL = {
     "sg_bbasis_rotate": 1, "sg_bidf": 3, "sg_bmask": 1,
     "sg_adjoint_stage1": 1, "sg_adjoint_stage2": 1, "sg_adjoint_stage3": 1, "sg_adjoint_final": 1,
     "sg_square_values": 1,
-    "sg_frag_count_lines": 4, "sg_frag_index_lines": 1, "sg_region_plan": 4, "sg_region_run": 5,
+    "sg_frag_count_lines": 4, "sg_frag_index_lines": 1, "sg_region_plan": 4, "sg_region_run": 5, "sg_region_index": 2, "sg_region_plan_indexed": 4, "sg_region_run_indexed": 5,
     "sg_csr_row_ptr": 4, "sg_csr_copy_rows": 1, "sg_gather_bytes": 1, "sg_nystrom_rescale": 1,
     "sg_sym_eig": 7, "sg_csr_aggregate_count": 2, "sg_csr_aggregate_run": 14,
 }

@@ -18,7 +18,7 @@ import torch
 
 from . import _lib
 from ._anndata import AnnData
-from ._binning import STRATEGIES, DeviceCSR
+from ._binning import STRATEGIES, DeviceCSR, emit_pairs
 
 
 def parse_region(s: str) -> tuple[str, int, int]:
@@ -83,41 +83,48 @@ def region_matrix(indptr: torch.Tensor, pos: torch.Tensor, length: torch.Tensor 
     F = int(pos.shape[0])
     st = STRATEGIES[strategy]
     names = list(chrom_sizes.names)
-    chrom_end = torch.from_numpy(np.cumsum(np.asarray(chrom_sizes.sizes, dtype=np.uint64)).view(np.int64)).to(dev)
-    excl = torch.tensor([1 if c in (exclude or ()) else 0 for c in names], dtype=torch.uint8, device=dev)
+    nc = len(names)
+    genome = int(np.sum(np.asarray(chrom_sizes.sizes, dtype=np.uint64), dtype=np.uint64))
+    table = np.empty(9 * nc, dtype=np.uint8)  # one copy for the two chromosome tables
+    table[:8 * nc] = np.cumsum(np.asarray(chrom_sizes.sizes, dtype=np.uint64)).view(np.uint8)
+    table[8 * nc:] = [c in (exclude or ()) for c in names]
+    table = torch.from_numpy(table).to(dev)
     if length is None:
         length = torch.zeros(max(F, 1), dtype=torch.int32, device=dev)
     mn = -1 if min_frag_size is None else int(min_frag_size)
     mx = -1 if max_frag_size is None else int(max_frag_size)
     nf = len(regions.names)
+    nr = int(regions.start.numel())
     sh = torch.cuda.current_stream(dev).cuda_stream
-    status = _lib.DeviceStatus(dev)
-    key_ptr = torch.empty(n + 1, dtype=torch.int64, device=dev)
     scan_scr = torch.empty(int(L.sg_scan_scratch_bytes(n + 1)), dtype=torch.uint8, device=dev)
-    rargs = [chrom_end.data_ptr(), excl.data_ptr(), len(names), regions.ptr.data_ptr(),
-             regions.start.data_ptr() if regions.start.numel() else None,
-             regions.end.data_ptr() if regions.end.numel() else None,
-             regions.maxend.data_ptr() if regions.maxend.numel() else None,
-             regions.rid.data_ptr() if regions.rid.numel() else None, nf, st, mn, mx]
-    _lib.check(L.sg_region_plan(indptr.data_ptr(), n, F, pos.data_ptr(), length.data_ptr(), *rargs,
-                                key_ptr.data_ptr(), scan_scr.data_ptr(), status.status_ptr, status.bad_ptr, sh),
+    nb = int(L.sg_region_index_bytes(genome, nr))
+    index = torch.empty(nb, dtype=torch.uint8, device=dev)
+    _lib.check(L.sg_region_index(genome, table.data_ptr(), nc, regions.ptr.data_ptr(),
+                                 regions.start.data_ptr() if nr else None, nr, index.data_ptr(), nb, sh),
+               "sg_region_index")
+    mask = torch.empty((F + 31) // 32 + 1, dtype=torch.int32, device=dev)
+    rargs = [table.data_ptr(), table.data_ptr() + 8 * nc, nc, regions.ptr.data_ptr(),
+             regions.start.data_ptr() if nr else None, regions.end.data_ptr() if nr else None,
+             regions.maxend.data_ptr() if nr else None, regions.rid.data_ptr() if nr else None, nf, st, mn, mx,
+             index.data_ptr(), genome, nr, mask.data_ptr()]
+    # [row pointers | status | lowest offending index]: one read gives the total and the status
+    plan = torch.empty(n + 3, dtype=torch.int64, device=dev)
+    status = _lib.DeviceStatus(dev, plan[n + 1:])
+    _lib.check(L.sg_region_plan_indexed(indptr.data_ptr(), n, F, pos.data_ptr(), length.data_ptr(), *rargs,
+                                        plan.data_ptr(), scan_scr.data_ptr(), status.status_ptr, status.bad_ptr, sh),
                "sg_region_plan")
-    status.raise_if_error("peak matrix: fragment position outside the genome", "fragment")
-    K = int(key_ptr[n].item()) if n > 0 else 0
+    K, *words = plan[n:].tolist()
+    status.raise_if(words, "peak matrix: fragment position outside the genome", "fragment")
     nbytes = int(L.sg_tile_scratch_bytes(K))
     scratch = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
-    out_indptr = torch.empty(n + 1, dtype=torch.int64, device=dev)
-    _lib.check(L.sg_region_run(indptr.data_ptr(), n, F, pos.data_ptr(), length.data_ptr(), *rargs,
-                               key_ptr.data_ptr(), scratch.data_ptr(), nbytes, out_indptr.data_ptr(),
-                               scan_scr.data_ptr(), status.status_ptr, status.bad_ptr, sh), "sg_region_run")
-    status.raise_if_error("peak matrix")
-    nnz = int(out_indptr[n].item()) if n > 0 else 0
-    out_idx = torch.empty(max(nnz, 1), dtype=torch.int32, device=dev)
-    out_cnt = torch.empty(max(nnz, 1), dtype=torch.int32, device=dev)
-    _lib.check(L.sg_tile_emit(n, key_ptr.data_ptr(), scratch.data_ptr(), nbytes, out_indptr.data_ptr(),
-                              out_idx.data_ptr(), out_cnt.data_ptr(), nnz, status.status_ptr, sh), "sg_tile_emit")
-    status.raise_if_error("peak matrix (emit)")
-    return DeviceCSR(out_indptr, out_idx[:nnz], out_cnt[:nnz], (n, nf))
+    out = torch.empty(n + 3, dtype=torch.int64, device=dev)
+    status = _lib.DeviceStatus(dev, out[n + 1:])
+    _lib.check(L.sg_region_run_indexed(indptr.data_ptr(), n, F, pos.data_ptr(), length.data_ptr(), *rargs,
+                                       plan.data_ptr(), scratch.data_ptr(), nbytes, out.data_ptr(),
+                                       scan_scr.data_ptr(), status.status_ptr, status.bad_ptr, sh), "sg_region_run")
+    nnz, *words = out[n:].tolist()
+    status.raise_if(words, "peak matrix")
+    return emit_pairs(plan, scratch, nbytes, out, n, nnz, status, nf, sh)
 
 
 def _peaks_from(adata, use_rep, peak_file):
