@@ -320,8 +320,10 @@ int sg_csr_select_cols(int64_t n, const int64_t* indptr, const int32_t* indices,
                        const int32_t* colmap, int64_t* out_indptr, int32_t* out_indices, float* out_values,
                        void* scan_scratch, void* stream);
 
-/* Number of row blocks used by sg_csr_transpose.                          */
+/* A number of row blocks for sg_csr_transpose that suits any matrix, and    */
+/* the one that suits n x m best (fewer blocks: less scratch).               */
 int sg_transpose_blocks(void);
+int sg_transpose_row_blocks(int64_t n, int64_t m);
 
 /* Bytes of scratch (256-B aligned) sg_csr_transpose needs.                 */
 int64_t sg_transpose_work_bytes(int64_t n, int64_t m, int nblk);

@@ -364,8 +364,7 @@ def transpose(csr: DeviceCSR, stream: int | None = None):
     n, m = csr.shape
     sh = torch.cuda.current_stream(dev).cuda_stream if stream is None else stream
     st = _lib.DeviceStatus(dev)
-    nblk = int(L.sg_transpose_blocks())
-    nblk = max(1, min(nblk, n))
+    nblk = int(L.sg_transpose_row_blocks(n, m))
     wbytes = int(L.sg_transpose_work_bytes(n, m, nblk))
     work = torch.empty(wbytes, dtype=torch.uint8, device=dev)
     colptr = torch.empty(m + 1, dtype=torch.int64, device=dev)

@@ -75,6 +75,7 @@ SIGNATURES: dict[str, tuple] = {
     "sg_radix_sort_u64": (_I32, [_I64, _P, _P, _P, _P, _I32, _I32, _P, _P, _P]),
     "sg_csr_select_cols": (_I32, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "sg_transpose_blocks": (_I32, []),
+    "sg_transpose_row_blocks": (_I32, [_I64, _I64]),
     "sg_transpose_work_bytes": (_I64, [_I64, _I64, _I32]),
     "sg_csr_transpose": (_I32, [_I64, _I64, _P, _P, _P, _I32, _P, _I64, _P, _P, _P, _P, _P, _P]),
     "sg_spectral_prepare": (_I32, [_I64, _I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,

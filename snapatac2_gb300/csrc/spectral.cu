@@ -12,6 +12,8 @@
 //   A v = a ⊙ (X (w² ⊙ (Xᵀ (a ⊙ v)))) - D⁻¹ ⊙ v
 // so X is kept as an index-only pattern (or with its integer counts) and the
 // scalings are folded into the SpMM prologue/epilogue.
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -62,81 +64,115 @@ __global__ void select_fill(int64_t n, const int64_t* __restrict__ ptr, const in
 // ---------------------------------------------------------------------------
 // deterministic transpose (CSR -> CSC) with rows ascending inside each column
 //
-// Columns are cut into panels of kTrPanel columns so that a CTA keeps the
-// counters / cursors of one panel in shared memory.  seg[r][p] is the offset
-// (from the row start) of row r's first entry in panel p (rows are sorted, so
-// a row's entries of one panel are contiguous).  Rows are split into nblk row
-// blocks; for every (row block, panel):
-//   count : shared-memory histogram of the panel's columns, written to
-//           cnt[b][col] (coalesced);
+// Columns are cut into panels of kTrPanel columns and rows into nblk blocks;
+// a CTA works on one (row block, panel).  seg[p][r] is the offset (from the
+// row start) of row r's first entry in panel p (rows are sorted, so a row's
+// entries of one panel are contiguous).
+//   count  : shared-memory histogram of the panel's columns, written to
+//            cnt[b][col] (coalesced);
 //   offsets: cnt[b][col] <- sum over earlier row blocks (column-wise scan);
-//   fill  : the CTA walks its rows in order and appends each row index to
-//           its column (one entry per column per row, so no two threads touch
-//           the same cursor inside a row; rows are separated by a barrier).
-// Row order inside every column is therefore ascending and the result is
-// identical run to run.
+//   fill   : kTrRows rows at a time, in any order within them: every entry
+//            sets its row's bit in its column's mask, and after a barrier its
+//            place is the column's cursor plus the number of lower bits set;
+//            then the cursors move and the masks are cleared.  Rows ascend in every column whatever order the threads run
+//            in, so the result is identical run to run.
+// What bounds it: about 17 entries per (row, panel) at 500,000 columns, so the
+// work is short segments of dependent loads and shared-memory atomics.  The
+// form before took the rows of a block one at a time with a barrier after
+// each (136 of 512 threads busy: 9.9 ms of fill, 4.3 of count) and 304 row
+// blocks (2.6 ms for the offsets).  Half a warp per row segment, three barriers
+// per 128 rows and some 20 row blocks take 5.0 ms (fill), 1.2 (count) and 1.1
+// (segments, before 2.1) at 100,000 x 500,000 and 4.1e8 nonzeros; the fill is
+// bound by its scattered 4-byte stores (L1 and L2 at two thirds).  2,048 columns per panel keep the partly written sectors of
+// all resident CTAs (four per SM) at 40 MB of the 129 MB of L2.
 // ---------------------------------------------------------------------------
-constexpr int kTrPanel = 16384;
+constexpr int kTrLog = 11;
+constexpr int kTrPanel = 1 << kTrLog;
+constexpr int kTrRows = 128;             // rows per step of the fill: four mask words per column
+constexpr int kTrThreads = 512;
+constexpr int kTrHalf = 16;              // lanes per row segment
+constexpr int kTrSlots = kTrThreads / kTrHalf;  // segments at a time
 
-__global__ void seg_kernel(int64_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, int pw,
-                           int P, int64_t m, int32_t* __restrict__ seg, int* status) {
+__global__ void seg_kernel(int64_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, int P,
+                           int64_t m, int32_t* __restrict__ seg, int* status) {
   const int lane = threadIdx.x & 31;
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t r = gw; r < n; r += nw) {
     const int64_t s = ptr[r], e = ptr[r + 1];
-    int32_t* sg = seg + r * (int64_t)(P + 1);
-    const int len = (int)(e - s);
-    for (int64_t k0 = s; k0 < e + 1; k0 += 32) {
-      const int64_t k = k0 + lane;
-      if (k > e) continue;
-      // panel of this entry (P for the end sentinel) and of the previous one
-      int pc = P, pp = -1;
-      if (k < e) {
-        const int c = idx[k];
-        if (c < 0 || c >= m || (k > s && idx[k - 1] >= c)) {  // need sorted, unique, in range
-          report_error(status, nullptr, SG_ERR_ARG, 0);
-          pc = P;
-        } else {
-          pc = c / pw;
+    int last = -1;  // column before this chunk
+    bool bad = false;
+    for (int64_t k0 = s; k0 < e; k0 += 64) {
+      const int64_t k1 = k0 + lane, k2 = k1 + 32;
+      const int c1 = k1 < e ? __ldg(idx + k1) : 0x7fffffff, c2 = k2 < e ? __ldg(idx + k2) : 0x7fffffff;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int64_t k = h ? k2 : k1;
+        const int c = h ? c2 : c1;
+        int prev = __shfl_up_sync(0xffffffffu, c, 1);
+        if (lane == 0) prev = last;
+        last = __shfl_sync(0xffffffffu, c, 31);
+        if (k < e) {
+          if (c < 0 || c >= m || prev >= c) {  // need sorted, unique, in range
+            bad = true;
+          } else {
+            const int pc = c >> kTrLog;
+            for (int p = (prev < 0 ? -1 : prev >> kTrLog) + 1; p <= pc; ++p) seg[(int64_t)p * n + r] = (int32_t)(k - s);
+          }
         }
       }
-      if (k > s) {
-        const int cprev = idx[k - 1];
-        pp = (cprev >= 0 && cprev < m) ? cprev / pw : P;
-      }
-      for (int p = pp + 1; p <= pc && p <= P; ++p) sg[p] = (int32_t)(k - s);
     }
-    if (len == 0 && lane == 0)
-      for (int p = 0; p <= P; ++p) sg[p] = 0;
+    if (bad) report_error(status, nullptr, SG_ERR_ARG, 0);
+    if (__any_sync(0xffffffffu, bad)) continue;  // seg is not read once the status is set
+    const int64_t tail = e > s ? (int64_t)(__ldg(idx + e - 1) >> kTrLog) + 1 : 0;
+    for (int64_t p = tail + lane; p <= P; p += 32) seg[p * n + r] = (int32_t)(e - s);
   }
 }
 
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(kTrThreads)
 tr_count(int64_t n, int64_t m, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-         const int32_t* __restrict__ seg, int P, int nblk, int32_t* __restrict__ cnt, const int* status) {
+         const int32_t* __restrict__ seg, int p0, int nblk, int32_t* __restrict__ cnt, const int* status) {
   __shared__ int32_t c_s[kTrPanel];
   if (*status) return;  // invalid column indices: seg is not trustworthy
-  const int b = blockIdx.x, p = blockIdx.y;
+  const int b = blockIdx.x, p = p0 + blockIdx.y;
   const int64_t r0 = n * b / nblk, r1 = n * (b + 1) / nblk;
-  const int64_t col0 = (int64_t)p * kTrPanel;
+  const int64_t col0 = (int64_t)p << kTrLog;
   const int width = (int)min((int64_t)kTrPanel, m - col0);
-  for (int j = threadIdx.x; j < width; j += blockDim.x) c_s[j] = 0;
+  for (int j = threadIdx.x; j < width; j += kTrThreads) c_s[j] = 0;
   __syncthreads();
-  for (int64_t r = r0; r < r1; ++r) {
-    const int32_t* sg = seg + r * (int64_t)(P + 1);
-    const int64_t s = ptr[r] + sg[p], e = ptr[r] + sg[p + 1];
-    for (int64_t k = s + threadIdx.x; k < e; k += blockDim.x) atomicAdd(&c_s[idx[k] - col0], 1);
+  const int32_t* lo = seg + (int64_t)p * n;
+  const int32_t* hi = lo + n;
+  const int l = threadIdx.x % kTrHalf;
+  int64_t r = r0 + threadIdx.x / kTrHalf;
+  int64_t s = 0, e = 0;
+  if (r < r1) {
+    const int64_t base = __ldg(ptr + r);
+    s = base + __ldg(lo + r);
+    e = base + __ldg(hi + r);
+  }
+  while (r < r1) {
+    const int64_t rn = r + kTrSlots;
+    int64_t sn = 0, en = 0;
+    if (rn < r1) {  // the next segment's bounds, in flight during this one
+      const int64_t base = __ldg(ptr + rn);
+      sn = base + __ldg(lo + rn);
+      en = base + __ldg(hi + rn);
+    }
+    for (int64_t k = s + l; k < e; k += kTrHalf) atomicAdd(&c_s[__ldg(idx + k) - (int)col0], 1);
+    r = rn;
+    s = sn;
+    e = en;
   }
   __syncthreads();
   int32_t* out = cnt + (int64_t)b * m + col0;
-  for (int j = threadIdx.x; j < width; j += blockDim.x) out[j] = c_s[j];
+  for (int j = threadIdx.x; j < width; j += kTrThreads) out[j] = c_s[j];
 }
 
 // colptr[j+1] = total count of column j
 __global__ void tr_total(int64_t m, int nblk, const int32_t* __restrict__ cnt, int64_t* __restrict__ colptr) {
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
     int64_t t = 0;
+#pragma unroll 8
     for (int b = 0; b < nblk; ++b) t += cnt[(int64_t)b * m + j];
     colptr[j + 1] = t;
     if (j == 0) colptr[0] = 0;
@@ -146,42 +182,104 @@ __global__ void tr_total(int64_t m, int nblk, const int32_t* __restrict__ cnt, i
 // cnt[b][j] <- sum_{b' < b} cnt[b'][j]  (row block b's offset inside column j)
 __global__ void tr_offsets(int64_t m, int nblk, int32_t* __restrict__ cnt) {
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
-    int64_t run = 0;
-    for (int b = 0; b < nblk; ++b) {
-      const int64_t c = cnt[(int64_t)b * m + j];
-      cnt[(int64_t)b * m + j] = (int32_t)run;
-      run += c;
+    int32_t run = 0;
+    for (int b0 = 0; b0 < nblk; b0 += 8) {  // eight loads in flight
+      int32_t c[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c[i] = b0 + i < nblk ? cnt[(int64_t)(b0 + i) * m + j] : 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (b0 + i < nblk) cnt[(int64_t)(b0 + i) * m + j] = run;
+        run += c[i];
+      }
     }
   }
 }
 
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(kTrThreads, 3)
 tr_fill(int64_t n, int64_t m, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-        const float* __restrict__ val, const int32_t* __restrict__ seg, int P, int nblk,
-        const int32_t* __restrict__ cnt, const int64_t* __restrict__ colptr, int32_t* __restrict__ rowidx,
-        float* __restrict__ cval, const int* status) {
-  __shared__ int32_t cur[kTrPanel];
+        const float* __restrict__ val, const int32_t* __restrict__ seg, int p0, int nblk,
+        const int32_t* __restrict__ cnt, const int64_t* __restrict__ colptr, int32_t* __restrict__ rowidx, float* __restrict__ cval,
+        const int* status) {
+  constexpr int W = kTrRows / 32;               // mask words per column
+  constexpr int R = kTrRows / kTrSlots;         // rows per half warp and step
+  extern __shared__ __align__(16) unsigned char tr_smem[];
+  int64_t* cur = reinterpret_cast<int64_t*>(tr_smem);                 // [kTrPanel] next place of the column
+  uint32_t(*mask)[kTrPanel] = reinterpret_cast<uint32_t(*)[kTrPanel]>(cur + kTrPanel);  // [W][kTrPanel]
   if (*status) return;
-  const int b = blockIdx.x, p = blockIdx.y;
+  const int b = blockIdx.x, p = p0 + blockIdx.y;
   const int64_t r0 = n * b / nblk, r1 = n * (b + 1) / nblk;
-  const int64_t col0 = (int64_t)p * kTrPanel;
+  const int64_t col0 = (int64_t)p << kTrLog;
   const int width = (int)min((int64_t)kTrPanel, m - col0);
   const int32_t* in = cnt + (int64_t)b * m + col0;
-  for (int j = threadIdx.x; j < width; j += blockDim.x) cur[j] = in[j];
+  for (int j = threadIdx.x; j < width; j += kTrThreads) {
+    cur[j] = colptr[col0 + j] + in[j];
+#pragma unroll
+    for (int w = 0; w < W; ++w) mask[w][j] = 0;
+  }
   __syncthreads();
-  for (int64_t r = r0; r < r1; ++r) {
-    const int32_t* sg = seg + r * (int64_t)(P + 1);
-    const int64_t s = ptr[r] + sg[p], e = ptr[r] + sg[p + 1];
-    for (int64_t k = s + threadIdx.x; k < e; k += blockDim.x) {
-      const int c = idx[k];
-      const int j = c - (int)col0;
-      const int pos = cur[j];
-      cur[j] = pos + 1;
-      const int64_t dst = colptr[c] + pos;
-      rowidx[dst] = (int32_t)r;
-      if (cval) cval[dst] = val[k];
+  const int32_t* lo = seg + (int64_t)p * n;
+  const int32_t* hi = lo + n;
+  const int l = threadIdx.x % kTrHalf, slot = threadIdx.x / kTrHalf;
+  auto place = [&](int j, int w, uint32_t bit) -> int {  // rows of this step below the entry's in its column
+    int below = 0;
+#pragma unroll
+    for (int v = 0; v < W; ++v) below += v <= w ? __popc(v < w ? mask[v][j] : mask[v][j] & (bit - 1u)) : 0;
+    return below;
+  };
+  for (int64_t q0 = r0; q0 < r1; q0 += kTrRows) {
+    int64_t s[R], e[R];
+    int c[R];  // the first piece of each segment stays in registers
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int64_t r = q0 + i * kTrSlots + slot;
+      s[i] = e[i] = 0;
+      if (r < r1) {
+        const int64_t base = __ldg(ptr + r);
+        s[i] = base + __ldg(lo + r);
+        e[i] = base + __ldg(hi + r);
+      }
     }
-    __syncthreads();  // the next row may touch the same columns
+#pragma unroll
+    for (int i = 0; i < R; ++i) c[i] = s[i] + l < e[i] ? __ldg(idx + s[i] + l) - (int)col0 : -1;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int t = i * kTrSlots + slot;
+      const uint32_t bit = 1u << (t & 31);
+      if (c[i] >= 0) atomicOr(&mask[t >> 5][c[i]], bit);
+      for (int64_t k = s[i] + l + kTrHalf; k < e[i]; k += kTrHalf)
+        atomicOr(&mask[t >> 5][__ldg(idx + k) - (int)col0], bit);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int t = i * kTrSlots + slot;
+      const uint32_t bit = 1u << (t & 31);
+      const int32_t row = (int32_t)(q0 + t);
+      if (c[i] >= 0) {
+        const int64_t dst = cur[c[i]] + place(c[i], t >> 5, bit);
+        rowidx[dst] = row;
+        if (cval) cval[dst] = val[s[i] + l];
+      }
+      for (int64_t k = s[i] + l + kTrHalf; k < e[i]; k += kTrHalf) {
+        const int j = __ldg(idx + k) - (int)col0;
+        const int64_t dst = cur[j] + place(j, t >> 5, bit);
+        rowidx[dst] = row;
+        if (cval) cval[dst] = val[k];
+      }
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < width; j += kTrThreads) {  // move the cursors past these rows
+      int t = 0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) t += __popc(mask[w][j]);
+      if (t) {
+        cur[j] += t;
+#pragma unroll
+        for (int w = 0; w < W; ++w) mask[w][j] = 0;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -245,10 +343,11 @@ __global__ void rownorm_kernel(int64_t n, const int64_t* __restrict__ ptr, const
   }
 }
 
-// colsum_j = w_j * sum_{i in col j} x_ij rinv_i   (CSC gather)
+// colsum_j = w_j * sum_{i in col j} x_ij rinv_i   (CSC gather); prod_j = w_j colsum_j
 __global__ void colsum_kernel(int64_t m, const int64_t* __restrict__ cptr, const int32_t* __restrict__ ridx,
                               const float* __restrict__ cval, const double* __restrict__ w,
-                              const double* __restrict__ rinv, double* __restrict__ colsum) {
+                              const double* __restrict__ rinv, double* __restrict__ colsum,
+                              double* __restrict__ prod) {
   const int lane = threadIdx.x & 31;
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -260,15 +359,20 @@ __global__ void colsum_kernel(int64_t m, const int64_t* __restrict__ cptr, const
       s += x;
     }
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) colsum[j] = s * w[j];
+    if (lane == 0) {
+      const double c = s * w[j];
+      colsum[j] = c;
+      prod[j] = w[j] * c;
+    }
   }
 }
 
-// d_i = rinv_i * sum_j x_ij w_j colsum_j ; dinv = 1/(d-1) ; a = rinv*sqrt(dinv)
+// d_i = rinv_i * sum_j x_ij prod_j ; dinv = 1/(d-1) ; a = rinv*sqrt(dinv).  The
+// gathers bind (one 32-byte sector of L2 per nonzero, one L1 lookup a clock):
+// one per nonzero instead of two, 2.62 -> 1.37 ms at 4.1e8 nonzeros.
 __global__ void degree_kernel(int64_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                              const float* __restrict__ val, const double* __restrict__ w,
-                              const double* __restrict__ colsum, const double* __restrict__ rinv,
-                              double* __restrict__ a, double* __restrict__ dinv, float* __restrict__ a32,
+                              const float* __restrict__ val, const double* __restrict__ prod,
+                              const double* __restrict__ rinv, double* __restrict__ a, double* __restrict__ dinv, float* __restrict__ a32,
                               float* __restrict__ dinv32, int* status, unsigned long long* bad) {
   const int lane = threadIdx.x & 31;
   const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -276,8 +380,7 @@ __global__ void degree_kernel(int64_t n, const int64_t* __restrict__ ptr, const 
   for (int64_t r = gw; r < n; r += nw) {
     double s = 0.0;
     for (int64_t k = ptr[r] + lane; k < ptr[r + 1]; k += 32) {
-      const int j = idx[k];
-      double x = w[j] * colsum[j];
+      double x = prod[idx[k]];
       if (val) x *= (double)val[k];
       s += x;
     }
@@ -498,6 +601,14 @@ extern "C" int sg_csr_select_cols(int64_t n, const int64_t* indptr, const int32_
 
 extern "C" int sg_transpose_blocks(void) { return 2 * sm_count(); }
 
+// Row blocks of a transpose: eight waves of the four CTAs that an SM holds,
+// and at least one step of the fill per block.
+extern "C" int sg_transpose_row_blocks(int64_t n, int64_t m) {
+  const int64_t P = (m + kTrPanel - 1) / kTrPanel;
+  const int64_t want = P > 0 ? (32 * (int64_t)sm_count() + P - 1) / P : 1, most = n / kTrRows;
+  return (int)std::max<int64_t>(1, std::min(want, most));
+}
+
 extern "C" int64_t sg_transpose_work_bytes(int64_t n, int64_t m, int nblk) {
   if (n < 0 || m <= 0 || nblk <= 0) return -1;
   const int64_t P = (m + kTrPanel - 1) / kTrPanel;
@@ -511,14 +622,19 @@ extern "C" int sg_csr_transpose(int64_t n, int64_t m, const int64_t* indptr, con
   if (n <= 0 || m <= 0 || nblk <= 0 || m > 0x7fffffffLL || n > 0x7fffffffLL) return SG_ERR_ARG;
   if (work_bytes < sg_transpose_work_bytes(n, m, nblk) || ((uintptr_t)work & 255u)) return SG_ERR_CAP;
   cudaStream_t s = as_stream(stream);
-  const int P = (int)((m + kTrPanel - 1) / kTrPanel);
+  const int64_t P64 = (m + kTrPanel - 1) / kTrPanel;
+  const int P = (int)P64;
   int32_t* cnt = reinterpret_cast<int32_t*>(work);
   int32_t* seg = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(work) + ((int64_t)nblk * m * 4 + 255) / 256 * 256);
-  seg_kernel<<<grid_for(n * 32, 256, 8 * sm_count() * 4), 256, 0, s>>>(n, indptr, indices, kTrPanel, P, m, seg,
-                                                                        status);
+  const size_t smem = kTrPanel * (sizeof(int64_t) + (kTrRows / 32) * sizeof(uint32_t));
+  if (cudaFuncSetAttribute(tr_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return SG_ERR_CUDA;
+  seg_kernel<<<grid_for(n * 32, 256, 8 * sm_count() * 4), 256, 0, s>>>(n, indptr, indices, P, m, seg, status);
   SG_CHECK_LAUNCH();
-  dim3 g2(nblk, P);
-  tr_count<<<g2, 512, 0, s>>>(n, m, indptr, indices, seg, P, nblk, cnt, status);
+  constexpr int kGridY = 32768;  // panels per launch (the grid's second dimension ends at 65,535)
+  for (int p0 = 0; p0 < P; p0 += kGridY)
+    tr_count<<<dim3(nblk, std::min(P - p0, kGridY)), kTrThreads, 0, s>>>(n, m, indptr, indices, seg, p0, nblk, cnt,
+                                                                         status);
   SG_CHECK_LAUNCH();
   const int g = grid_for(m, 256, 4096);
   tr_total<<<g, 256, 0, s>>>(m, nblk, cnt, colptr);
@@ -526,7 +642,9 @@ extern "C" int sg_csr_transpose(int64_t n, int64_t m, const int64_t* indptr, con
   if (inclusive_scan_i64(colptr + 1, m, scan_scratch, s) != cudaSuccess) return SG_ERR_CUDA;
   tr_offsets<<<g, 256, 0, s>>>(m, nblk, cnt);
   SG_CHECK_LAUNCH();
-  tr_fill<<<g2, 512, 0, s>>>(n, m, indptr, indices, values, seg, P, nblk, cnt, colptr, rowidx, cvalues, status);
+  for (int p0 = 0; p0 < P; p0 += kGridY)
+    tr_fill<<<dim3(nblk, std::min(P - p0, kGridY)), kTrThreads, smem, s>>>(n, m, indptr, indices, values, seg, p0, nblk,
+                                                                           cnt, colptr, rowidx, cvalues, status);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -553,11 +671,10 @@ extern "C" int sg_spectral_prepare(int64_t n, int64_t m, const int64_t* indptr, 
     idf_kernel<<<gm, 256, 0, s>>>(n, m, colptr, minmax, w);
     SG_CHECK_LAUNCH();
   }
-  square_weights<<<gm, 256, 0, s>>>(m, w, w2, w2_32);
   rownorm_kernel<<<gw_rows, 256, 0, s>>>(n, indptr, indices, values, w, rinv, status, bad);
-  colsum_kernel<<<gw_cols, 256, 0, s>>>(m, colptr, rowidx, cvalues, w, rinv, colsum);
-  degree_kernel<<<gw_rows, 256, 0, s>>>(n, indptr, indices, values, w, colsum, rinv, a, dinv, a32, dinv32,
-                                        status, bad);
+  colsum_kernel<<<gw_cols, 256, 0, s>>>(m, colptr, rowidx, cvalues, w, rinv, colsum, w2);  // w2 holds the product until it is set below
+  degree_kernel<<<gw_rows, 256, 0, s>>>(n, indptr, indices, values, w2, rinv, a, dinv, a32, dinv32, status, bad);
+  square_weights<<<gm, 256, 0, s>>>(m, w, w2, w2_32);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
