@@ -145,20 +145,20 @@ def import_device(d_text: torch.Tensor, chrom_sizes, *, min_num_fragments: int =
         cbase[1:] = np.cumsum(sizes[:-1], dtype=np.uint64)
     mito = {c.encode() if isinstance(c, str) else bytes(c) for c in (chrM or [])}
     cmito = np.array([n in mito for n in names], dtype=np.uint8)
-    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)  # noqa: E731
-    d_cblob, d_coff, d_size, d_base, d_mito = t(cblob), t(coff), t(sizes.view(np.int64)), t(cbase.view(np.int64)), t(cmito)
-
     has_wl = whitelist is not None
     wl = sorted({w.encode() if isinstance(w, str) else bytes(w) for w in whitelist}) if has_wl else []
     wblob, woff = _blob(wl)
-    d_wblob, d_woff = t(wblob), t(woff)
+    # the tables in one copy: 8-byte columns first, then the names, flags and barcodes
+    parts = [a.view(np.uint8) for a in (coff, sizes, cbase, woff, cblob, cmito, wblob)]
+    at = np.cumsum([0] + [a.size for a in parts])
+    d_tables = torch.from_numpy(np.concatenate(parts)).to(dev)
+    p_coff, p_size, p_base, p_woff, p_cblob, p_mito, p_wblob = (d_tables.data_ptr() + int(o) for o in at[:-1])
 
     ws_bytes = int(L.sg_frag_workspace_bytes(n_lines, len(wl)))
     ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
     info = (ctypes.c_int64 * 10)()
-    code = L.sg_frag_import(base, nbytes, line_start.data_ptr(), n_lines, d_cblob.data_ptr(), d_coff.data_ptr(),
-                            d_size.data_ptr(), d_base.data_ptr(), d_mito.data_ptr(), len(names),
-                            int(sizes.sum(dtype=np.uint64)), d_wblob.data_ptr(), d_woff.data_ptr(), len(wl),
+    code = L.sg_frag_import(base, nbytes, line_start.data_ptr(), n_lines, p_cblob, p_coff, p_size, p_base,
+                            p_mito, len(names), int(sizes.sum(dtype=np.uint64)), p_wblob, p_woff, len(wl),
                             int(has_wl), int(max(min_num_fragments, 0)), int(bool(sorted_by_barcode)),
                             int(shift_left), int(shift_right), HASH_SEED, ws.data_ptr(), ws_bytes, info, sh)
     inf = [int(v) for v in info]
