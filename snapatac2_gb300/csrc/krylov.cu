@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "small_chol.cuh"
 
 namespace sg {
 namespace {
@@ -155,58 +156,47 @@ __global__ void hrestart_kernel(double* __restrict__ H, int64_t ldh, int ld, int
   }
 }
 
-// Final correction sweep, small part (one CTA): G = RᵀR (Cholesky of the
-// symmetrised k x k Gram matrix), Ri = R⁻¹, C = Riᵀ sym(Hm) Ri.
-__global__ void refine_prep_kernel(int k, int kb, const double* __restrict__ G, const double* __restrict__ Hm,
-                                   double* __restrict__ Ri, double* __restrict__ C, double* __restrict__ tmp,
-                                   int* __restrict__ status) {
-  __shared__ double R[32][33];
-  __shared__ double I[32][33];
-  __shared__ int bad;
-  if (threadIdx.x == 0) {
-    bad = 0;
-    for (int j = 0; j < k && !bad; ++j) {
-      for (int c = j; c < k; ++c) {
-        double s = 0.5 * (G[j * kb + c] + G[c * kb + j]);
-        for (int i = 0; i < j; ++i) s -= R[i][j] * R[i][c];
-        if (c == j) {
-          if (!(s > 0.0)) { bad = 1; break; }
-          R[j][j] = sqrt(s);
-        } else {
-          R[j][c] = s / R[j][j];
-        }
-      }
-      for (int c = 0; c < j; ++c) R[j][c] = 0.0;
-    }
-    if (!bad) {  // inverse of the upper triangular R, column by column
-      for (int c = 0; c < k; ++c) {
-        for (int r = k - 1; r >= 0; --r) {
-          double s = r == c ? 1.0 : 0.0;
-          for (int q = r + 1; q < k; ++q) s -= R[r][q] * I[q][c];
-          I[r][c] = s / R[r][r];
-        }
-      }
-    } else {
-      atomicCAS(status, 0, SG_ERR_NUMERIC);
-    }
+// Final correction sweep, small part: G = RᵀR (Cholesky of the symmetrised
+// k x k Gram matrix), Ri = R⁻¹, C = Riᵀ sym(Hm) Ri.  One CTA per column of C:
+// each factors G for itself (the same operations, so the same factor), then
+// forms its column with four threads to an entry; CTA 0 writes Ri.  One thread
+// for the factor and the inverse and one CTA for the two products took
+// 1.8 ms at k = 30.
+__global__ void __launch_bounds__(kCholThreads)
+refine_prep_kernel(int k, int kb, const double* __restrict__ G, const double* __restrict__ Hm,
+                   double* __restrict__ Ri, double* __restrict__ C, int* __restrict__ status) {
+  __shared__ CholSmem<32> m;
+  __shared__ double x[32], y[32];
+  const int c = blockIdx.x;
+  for (int t = threadIdx.x; t < 32 * 32; t += kCholThreads) {
+    const int i = t / 32, j = t % 32;
+    m.a[i][j] = i < k && j < k ? 0.5 * (G[i * kb + j] + G[j * kb + i]) : 0.0;
+    m.a[i][32 + j] = i == j ? 1.0 : 0.0;
   }
+  chol_barrier();
+  if (!chol_inv<32>(k, m, 0.0)) {
+    if (c == 0 && threadIdx.x == 0) atomicCAS(status, 0, SG_ERR_NUMERIC);
+    return;
+  }
+  if (c == 0)
+    for (int t = threadIdx.x; t < k * k; t += kCholThreads) Ri[t] = t % k >= t / k ? m.r[t % k][32 + t / k] : 0.0;
+  // column c of Ri, y = sym(Hm) x, column c of C = Riᵀ y
+  if (threadIdx.x < 32) x[threadIdx.x] = (int)threadIdx.x <= c ? m.r[c][32 + threadIdx.x] : 0.0;
   __syncthreads();
-  if (bad) return;
-  for (int t = threadIdx.x; t < k * k; t += blockDim.x) Ri[t] = I[t / k][t % k];
-  // tmp = sym(Hm) Ri, C = Riᵀ tmp
-  for (int t = threadIdx.x; t < k * k; t += blockDim.x) {
-    const int r = t / k, c = t % k;
-    double s = 0.0;
-    for (int q = 0; q < k; ++q) s = fma(0.5 * (Hm[r * kb + q] + Hm[q * kb + r]), I[q][c], s);
-    tmp[t] = s;
-  }
+  const int r = threadIdx.x / 4, h = threadIdx.x % 4;
+  double s = 0.0;
+  if (r < k)
+    for (int q = h; q <= c; q += 4) s = fma(0.5 * (Hm[r * kb + q] + Hm[q * kb + r]), x[q], s);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if (h == 0) y[r] = s;
   __syncthreads();
-  for (int t = threadIdx.x; t < k * k; t += blockDim.x) {
-    const int r = t / k, c = t % k;
-    double s = 0.0;
-    for (int q = 0; q < k; ++q) s = fma(I[q][r], tmp[q * k + c], s);
-    C[t] = s;
-  }
+  s = 0.0;
+  if (r < k)
+    for (int q = h; q <= r; q += 4) s = fma(m.r[r][32 + q], y[q], s);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if (h == 0 && r < k) C[r * k + c] = s;
 }
 
 // Of the kr refined pairs (lam ascending, Z rows = eigenvectors of C) the k
@@ -267,7 +257,7 @@ struct Work {
   int64_t fx_bytes;
   RitzLayout ritz;
   // correction sweep
-  double *Up, *Zs64, *W64, *T64, *part32, *G32, *H32, *Ri, *Cs, *tmp, *Yr, *ev32;
+  double *Up, *Zs64, *W64, *T64, *part32, *G32, *H32, *Ri, *Cs, *Yr, *ev32;
   RitzLayout ritz32;
   int64_t bytes;
 };
@@ -292,13 +282,13 @@ Work layout(char* base, int code, int b, int k, int64_t n, int64_t m, int M, int
   const int64_t orl = take(rl.bytes);
   const bool refine = code == 0 && k <= 32;
   const int kb = 32;
-  int64_t oUp = 0, oZs64 = 0, oW64 = 0, oT64 = 0, op32 = 0, oG32 = 0, oH32 = 0, oRi32 = 0, oCs = 0, otmp = 0,
+  int64_t oUp = 0, oZs64 = 0, oW64 = 0, oT64 = 0, op32 = 0, oG32 = 0, oH32 = 0, oRi32 = 0, oCs = 0,
           oYr = 0, oev = 0, orl32 = 0;
   RitzLayout rl32{};
   if (refine) {
     oUp = take(n * kb * 8); oZs64 = take(n * kb * 8); oW64 = take(n * kb * 8); oT64 = take(m * kb * 8);
     op32 = take((int64_t)nparts * kb * kb * 8); oG32 = take(kb * kb * 8); oH32 = take(kb * kb * 8);
-    oRi32 = take(kb * kb * 8); oCs = take(kb * kb * 8); otmp = take(kb * kb * 8); oYr = take(kb * kb * 8);
+    oRi32 = take(kb * kb * 8); oCs = take(kb * kb * 8); oYr = take(kb * kb * 8);
     oev = take(kb * 8);
     rl32 = ritz_layout(nullptr, kb, kb);
     orl32 = take(rl32.bytes);
@@ -320,7 +310,7 @@ Work layout(char* base, int code, int b, int k, int64_t n, int64_t m, int M, int
     w.Up = (double*)(base + oUp); w.Zs64 = (double*)(base + oZs64); w.W64 = (double*)(base + oW64);
     w.T64 = (double*)(base + oT64); w.part32 = (double*)(base + op32); w.G32 = (double*)(base + oG32);
     w.H32 = (double*)(base + oH32); w.Ri = (double*)(base + oRi32); w.Cs = (double*)(base + oCs);
-    w.tmp = (double*)(base + otmp); w.Yr = (double*)(base + oYr); w.ev32 = (double*)(base + oev);
+    w.Yr = (double*)(base + oYr); w.ev32 = (double*)(base + oev);
     w.ritz32 = ritz_layout(base + orl32, kb, kb);
   }
   return w;
@@ -504,7 +494,7 @@ extern "C" int sg_lanczos(const sg_gram_op* op, int precision, int block, int k,
   auto cholqr2 = [&]() -> int {
     SG_TRY(sg_block_cholqr(code, b, n, w.W, w.part, nparts, w.G, w.R1, w.Rinv, status, s));
     SG_TRY(sg_block_cholqr(code, b, n, w.W, w.part, nparts, w.G, w.R2, w.Rinv, status, s));
-    nl += 8;
+    nl += b <= 8 ? 6 : 8;
     return SG_OK;
   };
   // start block: deterministic uniform noise, orthonormalised
@@ -619,7 +609,7 @@ extern "C" int sg_lanczos(const sg_gram_op* op, int precision, int block, int k,
       ++nl;
     }
     SG_TRY(sg_block_proj(1, kb, n, w.Up, kb, kb, w.W64, w.part32, nparts, w.H32, s));
-    refine_prep_kernel<<<1, 256, 0, s>>>(kr, kb, w.G32, w.H32, w.Ri, w.Cs, w.tmp, status);
+    refine_prep_kernel<<<kr, kCholThreads, 0, s>>>(kr, kb, w.G32, w.H32, w.Ri, w.Cs, status);
     SG_CHECK_LAUNCH();
     nl += 2 + 2 * proj_launches(1, kb, kb);
     int nw2 = 0;

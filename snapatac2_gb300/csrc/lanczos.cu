@@ -16,6 +16,7 @@
 //   rotate  out = Q[:, :m] Y                (thick restart, Ritz vectors)
 #include "common.cuh"
 #include "internal.h"
+#include "small_chol.cuh"
 
 namespace sg {
 namespace {
@@ -81,84 +82,223 @@ proj_partial(int64_t n, const T* __restrict__ Q, int64_t ldq, int ncols, const T
   }
 }
 
-// Gram partials of a block: part[blk][i*B + j] = sum over this CTA's rows of
-// W[r,i] W[r,j].  Thread per row (all threads busy, unlike the projection
-// kernel with only B basis columns); upper triangle in registers, then a
-// fixed-order reduction over the CTA's threads (deterministic).
-template <typename T, int B>
-__global__ void __launch_bounds__(256) gram_partial(int64_t n, const T* __restrict__ W, double* __restrict__ part) {
-  constexpr int NT = B * (B + 1) / 2;
-  __shared__ double red[256 / 32][NT];
+// ---- Gram matrix of a block of 4 or 8 ----------------------------------------
+// part[blk][t] = sum over this CTA's rows of W[r,i] W[r,j], t = the packed
+// upper triangle (i <= j).  Fixed orders throughout: deterministic.  At 5,000
+// rows the reduction of the 36 sums over a warp's lanes, 5 additions each on
+// the FP64 pipe (about two lanes per clock per SM, idle lanes and warps
+// included), had all of the time: 31 us a launch, eight warps for 17 rows
+// (now 3.7 us in FP64; FP32 at 30,000 rows 32 -> 7.4 us).
+constexpr int kGramRows = 64;  // rows per CTA at least, where the grid allows
+
+template <int B>
+__host__ __device__ constexpr int tri_count() { return B * (B + 1) / 2; }
+
+// position t of the packed upper triangle -> (i, j)
+template <int B>
+__device__ __forceinline__ void tri_pos(int t, int& i, int& j) {
+  i = 0;
+  while (t >= B - i) { t -= B - i; ++i; }
+  j = i + t;
+}
+
+// FP64: a thread owns one entry and every kRG-th row, so that a row costs
+// tri_count / 32 warp instructions and nothing is left to reduce but the kRG
+// partial sums of an entry (8 x 36 = 288 threads for blocks of 8, 16 x 10 =
+// 160 for blocks of 4: whole warps, no idle lanes).
+template <int B>
+__host__ __device__ constexpr int gram_groups() { return B == 8 ? 8 : 16; }
+
+template <int B>
+__global__ void __launch_bounds__(tri_count<B>() * gram_groups<B>())
+gram_entries(int64_t n, const double* __restrict__ W, double* __restrict__ part) {
+  constexpr int NT = tri_count<B>(), RG = gram_groups<B>(), U = 4;
+  __shared__ double red[RG][NT];
   const int nb = gridDim.x, b = blockIdx.x;
   const int64_t r0 = n * b / nb, r1 = n * (b + 1) / nb;
-  T acc[NT];
+  const int t = threadIdx.x % NT, g = threadIdx.x / NT;
+  int i, j;
+  tri_pos<B>(t, i, j);
+  double acc = 0.0;
+  int64_t r = r0 + g;
+  for (; r + (U - 1) * RG < r1; r += U * RG) {  // several rows' loads in flight
+    double x[U], y[U];
 #pragma unroll
-  for (int t = 0; t < NT; ++t) acc[t] = T(0);
-  for (int64_t r = r0 + threadIdx.x; r < r1; r += 256) {
-    T w[B];
+    for (int u = 0; u < U; ++u) {
+      x[u] = W[(r + u * RG) * B + i];
+      y[u] = W[(r + u * RG) * B + j];
+    }
 #pragma unroll
-    for (int i = 0; i < B; ++i) w[i] = W[r * B + i];
-    int t = 0;
-#pragma unroll
-    for (int i = 0; i < B; ++i)
-#pragma unroll
-      for (int j = i; j < B; ++j) {
-        acc[t] = fma(w[i], w[j], acc[t]);
-        ++t;
-      }
+    for (int u = 0; u < U; ++u) acc = fma(x[u], y[u], acc);
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    double v = (double)acc[t];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[wid][t] = v;
-  }
+  for (; r < r1; r += RG) acc = fma(W[r * B + i], W[r * B + j], acc);
+  red[g][t] = acc;
   __syncthreads();
-  for (int t = threadIdx.x; t < NT; t += 256) {
+  if (g == 0) {
     double v = 0.0;
-    for (int w2 = 0; w2 < 256 / 32; ++w2) v += red[w2][t];
-    // position t -> (i, j) of the packed upper triangle
-    int i = 0, rem = t;
-    while (rem >= B - i) { rem -= B - i; ++i; }
-    const int j = i + rem;
-    part[(int64_t)b * B * B + i * B + j] = v;
-    part[(int64_t)b * B * B + j * B + i] = v;
+#pragma unroll
+    for (int q = 0; q < RG; ++q) v += red[q][t];
+    part[(int64_t)b * NT + t] = v;
   }
 }
 
+// FP32: a thread per row, the products and a thread's own rows in FP32, the
+// sums over threads in FP64 by transpose butterflies (32 of the 36 sums take
+// 31 additions, not 160), and none in warps that have no row.
+template <int B>
+__global__ void __launch_bounds__(256) gram_rows(int64_t n, const float* __restrict__ W, double* __restrict__ part) {
+  constexpr int NT = tri_count<B>();
+  constexpr int kMain = B == 8 ? 32 : 8, kRest = NT - kMain;  // 32 + 4, 8 + 2
+  __shared__ double red[256 / 32][NT];
+  const int nb = gridDim.x, b = blockIdx.x;
+  const int64_t r0 = n * b / nb, r1 = n * (b + 1) / nb;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int live = (int)(r1 - r0 < 256 ? (r1 - r0 + 31) / 32 : 8);  // warps with a row
+  if (wid < live) {
+    float acc[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) acc[t] = 0.f;
+    for (int64_t r = r0 + threadIdx.x; r < r1; r += 256) {
+      float w[B];
+#pragma unroll
+      for (int i = 0; i < B; ++i) w[i] = W[r * B + i];
+      int t = 0;
+#pragma unroll
+      for (int i = 0; i < B; ++i)
+#pragma unroll
+        for (int j = i; j < B; ++j) {
+          acc[t] = fmaf(w[i], w[j], acc[t]);
+          ++t;
+        }
+    }
+    double m[kMain], e[kRest];
+#pragma unroll
+    for (int t = 0; t < kMain; ++t) m[t] = (double)acc[t];
+#pragma unroll
+    for (int t = 0; t < kRest; ++t) e[t] = (double)acc[kMain + t];
+    warp_colsum<double, kMain>(m, lane);
+    warp_colsum<double, kRest>(e, lane);
+    // sum c of C ends in the lanes whose high bits spell c
+    if (lane % (32 / kMain) == 0) red[wid][lane / (32 / kMain)] = m[0];
+    if (lane % (32 / kRest) == 0) red[wid][kMain + lane / (32 / kRest)] = e[0];
+  }
+  __syncthreads();
+  if (threadIdx.x < NT) {
+    double v = 0.0;
+    for (int w2 = 0; w2 < live; ++w2) v += red[w2][threadIdx.x];
+    part[(int64_t)b * NT + threadIdx.x] = v;
+  }
+}
+
+// G = sum of the nb packed partials, then G = RᵀR and R⁻¹ (small_chol.cuh):
+// one CTA, 8 (blocks of 4: 16) threads per entry for the sum in a fixed
+// order, four warps for the factor.  A non-positive pivot relative to the
+// diagonal sets SG_ERR_NUMERIC (rank-deficient block).  7.2 us a launch for 79
+// partials (5,000 rows); the sum and the factor as two launches took 17 us.
+constexpr double kCholTol = 1e-28;
+
+template <int P>
+__device__ void write_factor(int B, const CholSmem<P>& m, bool ok, double* __restrict__ R, double* __restrict__ Rinv,
+                             int* status) {
+  for (int t = threadIdx.x; t < B * B; t += kCholThreads) {
+    const int i = t / B, j = t % B;
+    R[t] = j >= i ? m.r[i][j] : 0.0;
+    Rinv[t] = j >= i ? m.r[j][P + i] : 0.0;
+  }
+  if (!ok && threadIdx.x == 0) atomicCAS(status, 0, SG_ERR_NUMERIC);
+}
+
+template <int B>
+__global__ void __launch_bounds__(tri_count<B>() * gram_groups<B>())
+gram_chol(int nb, const double* __restrict__ part, double* __restrict__ G, double* __restrict__ R,
+          double* __restrict__ Rinv, int* status) {
+  constexpr int NT = tri_count<B>(), RG = gram_groups<B>(), U = 8;
+  static_assert(NT * RG >= kCholThreads, "the factor needs four warps");
+  __shared__ double red[RG][NT];
+  __shared__ CholSmem<B> m;
+  const int t = threadIdx.x % NT, g = threadIdx.x / NT;
+  double s = 0.0;
+  int q = g;
+  for (; q + (U - 1) * RG < nb; q += U * RG) {
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = part[(int64_t)(q + u * RG) * NT + t];
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += v[u];
+  }
+  for (; q < nb; q += RG) s += part[(int64_t)q * NT + t];
+  red[g][t] = s;
+  __syncthreads();
+  if (threadIdx.x >= kCholThreads) return;
+  for (int x = threadIdx.x; x < B * B; x += kCholThreads) m.a[x / B][B + x % B] = x / B == x % B ? 1.0 : 0.0;
+  if (threadIdx.x < NT) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < RG; ++w) v += red[w][threadIdx.x];
+    int i, j;
+    tri_pos<B>(threadIdx.x, i, j);
+    m.a[i][j] = v;
+    m.a[j][i] = v;
+    G[i * B + j] = v;
+    G[j * B + i] = v;
+  }
+  chol_barrier();
+  const bool ok = chol_inv<B>(B, m, kCholTol);
+  write_factor<B>(B, m, ok, R, Rinv, status);
+}
+
+// The factor alone, of a Gram matrix already summed (blocks of 16 and 32).
+template <int P>
+__global__ void __launch_bounds__(kCholThreads)
+chol_kernel(const double* __restrict__ G, double* __restrict__ R, double* __restrict__ Rinv, int* status) {
+  __shared__ CholSmem<P> m;
+  for (int x = threadIdx.x; x < P * P; x += kCholThreads) {
+    m.a[x / P][x % P] = G[x];
+    m.a[x / P][P + x % P] = x / P == x % P ? 1.0 : 0.0;
+  }
+  chol_barrier();
+  const bool ok = chol_inv<P>(P, m, kCholTol);
+  write_factor<P>(P, m, ok, R, Rinv, status);
+}
+
 // C[t] = sum over the nparts partials of part[b][t], t < tot = ncols * B.  A
-// CTA owns 32 consecutive outputs (lane = output, coalesced reads); warp w
-// sums the partials b = w, w + 32, ... in order, then the 32 warp sums are
-// added in warp order: a fixed order, so the result is deterministic.
-constexpr int kReduceWarps = 32;
-__global__ void __launch_bounds__(kReduceWarps * 32)
+// CTA owns 8 consecutive outputs (64-byte reads): its 32 groups of 8 lanes
+// take the partials b = g, g + 32, ... in order, then the four groups of a
+// warp and the eight warps are added in a fixed order, so the result is
+// deterministic.  What it costs is the FP64 additions of one CTA (about two
+// lanes per clock per SM): with 32 outputs to a CTA of 1,024 threads a launch
+// over 304 partials took 6 us, on as few as two SMs; now 3.5 us.
+constexpr int kReduceOut = 8;
+constexpr int kReduceThreads = 256;
+__global__ void __launch_bounds__(kReduceThreads)
 proj_reduce(int nparts, int ncols, int B, const double* __restrict__ part, double* __restrict__ C) {
-  __shared__ double ws[kReduceWarps][33];
+  constexpr int kGroups = kReduceThreads / kReduceOut, U = 5;
+  __shared__ double ws[kReduceThreads / 32][kReduceOut];
   const int tot = ncols * B;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int t = blockIdx.x * 32 + lane;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = threadIdx.x / kReduceOut;
+  const int t = blockIdx.x * kReduceOut + threadIdx.x % kReduceOut;
   double s = 0.0;
   if (t < tot) {
-    int b = w;
-    for (; b + 3 * kReduceWarps < nparts; b += 4 * kReduceWarps) {
-      const double v0 = part[(int64_t)b * tot + t], v1 = part[(int64_t)(b + kReduceWarps) * tot + t];
-      const double v2 = part[(int64_t)(b + 2 * kReduceWarps) * tot + t];
-      const double v3 = part[(int64_t)(b + 3 * kReduceWarps) * tot + t];
-      s += v0;
-      s += v1;
-      s += v2;
-      s += v3;
+    int b = g;
+    for (; b + (U - 1) * kGroups < nparts; b += U * kGroups) {
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = part[(int64_t)(b + u * kGroups) * tot + t];
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += v[u];
     }
-    for (; b < nparts; b += kReduceWarps) s += part[(int64_t)b * tot + t];
+    for (; b < nparts; b += kGroups) s += part[(int64_t)b * tot + t];
   }
-  ws[w][lane] = s;
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  if (lane < kReduceOut) ws[w][lane] = s;
   __syncthreads();
-  if (w == 0 && t < tot) {
-    double r = 0.0;
-    for (int k = 0; k < kReduceWarps; ++k) r += ws[k][lane];
-    C[t] = r;
+  if (w == 0) {  // lane = (pair of warps, output)
+    const int o = lane % kReduceOut, h = lane / kReduceOut;
+    double r = ws[2 * h][o] + ws[2 * h + 1][o];
+    r += __shfl_xor_sync(0xffffffffu, r, 8);
+    r += __shfl_xor_sync(0xffffffffu, r, 16);
+    if (lane < kReduceOut && t < tot) C[t] = r;
   }
 }
 
@@ -492,63 +632,6 @@ bool tiled_ok(const void* Q, int64_t ldq, const void* W) {
   return ((uintptr_t)Q & 15u) == 0 && ((uintptr_t)W & 15u) == 0 && (ldq & 3) == 0;
 }
 
-// Cholesky of the B x B Gram matrix (one warp, lane j owns column j):
-// G = RᵀR with R upper triangular; also Rinv = R⁻¹.  A non-positive pivot
-// relative to the diagonal sets SG_ERR_NUMERIC (rank-deficient block).  G is
-// staged in shared memory first; lane j's column of R⁻¹ is built in shared
-// memory (no per-thread local arrays).
-__global__ void chol_kernel(int B, const double* __restrict__ G, double* __restrict__ R,
-                            double* __restrict__ Rinv, int* status) {
-  // FP64 divisions and square roots are long dependent chains on GB300's
-  // FP64 unit: each pivot takes one reciprocal square root (r_kk = s·rsqrt(s),
-  // 1/r_kk = rsqrt(s)) and every division becomes a product with it
-  __shared__ double g[32][33];
-  __shared__ double r[32][33];
-  __shared__ double x[32][33];  // x[i][j]: row i of column j of R⁻¹
-  __shared__ double rd[32];     // 1 / r[k][k]
-  const int j = threadIdx.x;
-  for (int t = j; t < B * B; t += 32) g[t / B][t % B] = G[t];
-  for (int i = 0; i < B; ++i) {
-    r[i][j] = 0.0;
-    x[i][j] = 0.0;
-  }
-  __syncwarp();
-  bool fail = false;
-  for (int k = 0; k < B; ++k) {
-    if (j == k) {
-      double s = g[k][k];
-      for (int i = 0; i < k; ++i) s -= r[i][k] * r[i][k];
-      const double gkk = g[k][k];
-      if (!(s > 1e-28 * (gkk > 0 ? gkk : 1.0)) || !(s > 0.0)) { fail = true; s = 1.0; }
-      const double rs = rsqrt(s);
-      r[k][k] = s * rs;
-      rd[k] = rs;
-    }
-    __syncwarp();
-    const double ip = rd[k];
-    if (j > k && j < B) {
-      double s = g[k][j];
-      for (int i = 0; i < k; ++i) s -= r[i][k] * r[i][j];
-      r[k][j] = s * ip;
-    }
-    __syncwarp();
-  }
-  if (__any_sync(0xffffffffu, fail) && j == 0) atomicCAS(status, 0, SG_ERR_NUMERIC);
-  // back substitution, lane j computes column j of R^-1
-  if (j < B) {
-    x[j][j] = rd[j];
-    for (int i = j - 1; i >= 0; --i) {
-      double s = 0.0;
-      for (int t = i + 1; t <= j; ++t) s += r[i][t] * x[t][j];
-      x[i][j] = -s * rd[i];
-    }
-    for (int i = 0; i < B; ++i) {
-      Rinv[i * B + j] = i <= j ? x[i][j] : 0.0;
-      R[i * B + j] = r[i][j];
-    }
-  }
-}
-
 // W[i,:] <- W[i,:] Rinv, FP32 blocks of 16: thread per row, the row in
 // registers, Rinv in shared memory read as broadcasts; column c sums
 // W[i,k] Rinv[k,c] over k = 0..c in order (the order of the warp form)
@@ -725,7 +808,7 @@ int proj_tiled_launch(int64_t n, const float* Q, int64_t ldq, int ncols, const f
     return SG_ERR_CUDA;
   proj_tiled<B><<<nparts, kTileWarps * 32, smem, s>>>(n, Q, ldq, ncols, W, part);
   SG_CHECK_LAUNCH();
-  proj_reduce<<<(ncols * B + 31) / 32, kReduceWarps * 32, 0, s>>>(nparts, ncols, B, part, C);
+  proj_reduce<<<(ncols * B + kReduceOut - 1) / kReduceOut, kReduceThreads, 0, s>>>(nparts, ncols, B, part, C);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -750,7 +833,7 @@ int proj_t(int64_t n, const T* Q, int64_t ldq, int ncols, const T* W, double* pa
     }
     SG_CHECK_LAUNCH();
     const int tot = nc * B;
-    proj_reduce<<<(tot + 31) / 32, kReduceWarps * 32, 0, s>>>(nparts, nc, B, part, C + (int64_t)c0 * B);
+    proj_reduce<<<(tot + kReduceOut - 1) / kReduceOut, kReduceThreads, 0, s>>>(nparts, nc, B, part, C + (int64_t)c0 * B);
     SG_CHECK_LAUNCH();
   }
   return SG_OK;
@@ -885,21 +968,31 @@ extern "C" int sg_block_update(int dtype, int block, int64_t n, const void* Q, i
 // One Cholesky-QR pass: G = WᵀW, G = RᵀR, W <- W R⁻¹.  G, R, Rinv: B x B FP64.
 extern "C" int sg_block_cholqr(int dtype, int block, int64_t n, void* W, double* part, int nparts, double* G,
                                double* R, double* Rinv, int* status, void* stream) {
-  if (n <= 0 || block < 1 || block > 32) return SG_ERR_ARG;
+  if (n <= 0 || nparts <= 0 || (dtype != 0 && dtype != 1)) return SG_ERR_ARG;
   cudaStream_t s = as_stream(stream);
-  int e = SG_OK;
-  if (dtype == 0 && block == 8) gram_partial<float, 8><<<nparts, 256, 0, s>>>(n, (const float*)W, part);
-  else if (dtype == 0 && block == 4) gram_partial<float, 4><<<nparts, 256, 0, s>>>(n, (const float*)W, part);
-  else if (dtype == 1 && block == 8) gram_partial<double, 8><<<nparts, 256, 0, s>>>(n, (const double*)W, part);
-  else if (dtype == 1 && block == 4) gram_partial<double, 4><<<nparts, 256, 0, s>>>(n, (const double*)W, part);
-  else e = sg_block_proj(dtype, block, n, W, block, block, W, part, nparts, G, stream);
-  if (e) return e;
   if (block == 4 || block == 8) {
-    SG_CHECK_LAUNCH();
-    proj_reduce<<<(block * block + 31) / 32, kReduceWarps * 32, 0, s>>>(nparts, block, block, part, G);
-    SG_CHECK_LAUNCH();
+    // the packed partials take less room than the projection's (part holds
+    // nparts x block x block); no more CTAs than have kGramRows rows each:
+    // the one CTA that adds them up pays for each
+    const int64_t want = (n + kGramRows - 1) / kGramRows;
+    const int nb = (int)(want < nparts ? want : nparts);
+    if (block == 8) {
+      if (dtype == 0) gram_rows<8><<<nb, 256, 0, s>>>(n, (const float*)W, part);
+      else gram_entries<8><<<nb, tri_count<8>() * gram_groups<8>(), 0, s>>>(n, (const double*)W, part);
+      SG_CHECK_LAUNCH();
+      gram_chol<8><<<1, tri_count<8>() * gram_groups<8>(), 0, s>>>(nb, part, G, R, Rinv, status);
+    } else {
+      if (dtype == 0) gram_rows<4><<<nb, 256, 0, s>>>(n, (const float*)W, part);
+      else gram_entries<4><<<nb, tri_count<4>() * gram_groups<4>(), 0, s>>>(n, (const double*)W, part);
+      SG_CHECK_LAUNCH();
+      gram_chol<4><<<1, tri_count<4>() * gram_groups<4>(), 0, s>>>(nb, part, G, R, Rinv, status);
+    }
+  } else {
+    const int e = sg_block_proj(dtype, block, n, W, block, block, W, part, nparts, G, stream);
+    if (e) return e;
+    if (block == 16) chol_kernel<16><<<1, kCholThreads, 0, s>>>(G, R, Rinv, status);
+    else chol_kernel<32><<<1, kCholThreads, 0, s>>>(G, R, Rinv, status);
   }
-  chol_kernel<<<1, 32, 0, s>>>(block, G, R, Rinv, status);
   SG_CHECK_LAUNCH();
   if (dtype == 0) return rinv_dispatch<float>(block, n, Rinv, (float*)W, s);
   if (dtype == 1) return rinv_dispatch<double>(block, n, Rinv, (double*)W, s);
