@@ -161,7 +161,7 @@ class LanczosInfo(ctypes.Structure):
                 ("spmm_launches", _I64), ("kernel_launches", _I64)]
 
 # Kernels launched by one call of each entry point (launch accounting of the
-# benchmark): e.g. sg_block_cholqr = projection partial + reduce + Cholesky +
+# benchmark): e.g. sg_block_cholqr = Gram partials + their sum and Cholesky +
 # R⁻¹ application.
 KERNELS_PER_CALL = {
     "sg_tile_plan": 4, "sg_tile_bound": 1, "sg_tile_run": 5, "sg_tile_emit": 1, "sg_col_counts": 2, "sg_csr_select_cols": 5,
@@ -174,7 +174,7 @@ KERNELS_PER_CALL = {
     "sg_square_values": 1,
     "sg_frag_count_lines": 4, "sg_frag_index_lines": 1, "sg_region_plan": 4, "sg_region_run": 5, "sg_region_index": 2, "sg_region_plan_indexed": 4, "sg_region_run_indexed": 5,
     "sg_csr_row_ptr": 4, "sg_csr_copy_rows": 1, "sg_gather_bytes": 1, "sg_nystrom_rescale": 1,
-    "sg_sym_eig": 7, "sg_csr_aggregate_count": 2, "sg_csr_aggregate_run": 14,
+    "sg_sym_eig": 11, "sg_csr_aggregate_count": 2, "sg_csr_aggregate_run": 14,
 }
 
 _lock = threading.Lock()

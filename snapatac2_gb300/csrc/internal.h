@@ -35,7 +35,9 @@ struct RitzLayout {
   double* Zt;          // eigenvectors of the selected ones (rows)
   double* lu;          // inverse-iteration scratch
   unsigned char* piv;  //
-  double* G;           // Gram matrix of the selected vectors (Cholesky-QR)
+  double* G;           // Gram matrix of the selected vectors, less the identity
+  double* T;           // triangular factors of the blocks of reflectors
+  int* wide;           // nonzero: the vectors are far from orthonormal
   int64_t bytes;
 };
 RitzLayout ritz_layout(char* base, int n, int nw);

@@ -9,9 +9,9 @@
 //
 //   tridiag    Householder reduction A = Q T Qᵀ on one thread-block cluster
 //              (up to 16 CTAs).  Row i of A lives in the shared memory of CTA
-//              i mod CS; each step broadcasts the reflector and the product
-//              p = τ A v through distributed shared memory, with two cluster
-//              barriers per step (buffers alternate between steps).
+//              i mod CS; each step passes the product A v on through
+//              distributed shared memory, with one cluster barrier per step
+//              (buffers alternate between steps).
 //   bisect     eigenvalues of T by multisection on Sturm counts: one warp per
 //              wanted eigenvalue, 32 shifts per round, to absolute accuracy
 //              eps·‖T‖ (LAPACK dstebz's default).
@@ -19,13 +19,16 @@
 //              tridiagonal LU (as LAPACK dstein): one warp per cluster of
 //              near-degenerate eigenvalues (1e-9 ‖T‖), modified Gram-Schmidt
 //              inside a cluster.
-//   orth       one FP64 Cholesky-QR of all the vectors (Gram matrix by
-//              warps across the GPU, factor and triangular solve in one CTA):
-//              separately iterated vectors of eigenvalues 1e-9..1e-3 ‖T‖
-//              apart are orthogonal only to eps ‖T‖ / gap; rotating them by
-//              that much moves their residuals by ~eps ‖T‖.
-//   backtr     eigenvectors of A = Q z: one warp per vector applies the
-//              reflectors in reverse order.
+//   backtr     eigenvectors of A = Q z: one CTA per vector applies the
+//              reflectors in reverse order, eight at a time.
+//   orth       all the vectors to the closest orthonormal set: separately
+//              iterated vectors of eigenvalues 1e-9..1e-3 ‖T‖ apart are
+//              orthogonal only to eps ‖T‖ / gap; moving them by that much
+//              moves their residuals by ~eps ‖T‖.  Two steps of a quadratic
+//              iteration spread over the GPU (0.26 ms for 288 vectors of
+//              length 336; a Cholesky-QR with its factor on one CTA took 7.0);
+//              vectors too far off for it (an inverse iteration that did not
+//              converge) still take the Cholesky-QR.
 //
 // Every sum runs in a fixed order, so results are reproducible run to run.
 #include <cooperative_groups.h>
@@ -50,151 +53,183 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// Shared memory of the reduction: rows [R][n], v[2][n], p[2][n], 2 x 32
-// slots (per-CTA partial sums of pᵀv in 0..CS-1, τ in 16), 32 per-warp
-// partials, 4 scalars.  v and the slots are double-buffered: the owner of
-// step j + 1 writes them into the other CTAs before those have finished step
-// j.  p is written by the other CTAs only after the step's first cluster
-// barrier, so the p buffer of the other parity holds w = p + K v.
+// Shared memory of the reduction: rows [R][n], v[2][n], u[2][n], 2 x
+// kMaxCluster x kTriWarps partial sums of uᵀv, one per warp of the cluster,
+// per-warp partials, 8 scalars.
+constexpr int kTriWarps = kTriThreads / 32;
 inline size_t tridiag_smem(int n, int CS) {
   const int R = (n + CS - 1) / CS;
-  return ((size_t)R * n + 4 * (size_t)n + 64 + 32 + 4) * sizeof(double);
+  return ((size_t)R * n + 4 * (size_t)n + 2 * kMaxCluster * kTriWarps + kTriWarps + 8) * sizeof(double);
 }
 
-// GB300 runs FP64 at about two lanes per clock per SM, so a warp-wide FP64
-// instruction holds its SM sub-partition for tens of clocks: the scalar steps
-// (the reflector's norm, square root and divisions, the K factor) run once,
-// on one thread or one warp, and are passed on through shared memory; the
-// vector w = p + K v is formed once per step, and each trailing element is
-// updated by two FMAs.
+// GB300 runs FP64 at about two lanes per clock per SM: a warp-wide FP64
+// instruction holds its SM sub-partition for 64 clocks and the next one that
+// needs its result waits longer, so a step costs its FP64 work plus a chain of
+// dependent operations.  One cluster barrier per step: step j
+//   1. forms w = τ u + K v of the reflector before it (u = A v arrived over
+//      distributed shared memory in step j - 1, K = -τ² uᵀv / 2 from the
+//      warps' partial sums),
+//   2. pulls row j from its owner, applies that reflector to it and finds
+//      reflector j from the result -- in every CTA, with the same operations,
+//      so nothing is broadcast,
+//   3. applies the rank-2 update to the rows this CTA owns and multiplies them
+//      by the new v in the same pass, and sends the products to every CTA.
+// The reflector is not scaled to a unit first element (H = I - τ v vᵀ with
+// τ = 1 / (μ (μ + |α|)), μ the norm of the row's part below the diagonal), so
+// the matrix pass starts after one square root; the reciprocal for τ, first
+// used in the next step, runs beside the pass.  With the reflector made by the
+// owner and broadcast, and the update and the product as two passes between
+// two cluster barriers, a step at n = 336 took 7.9 us; it takes 6.6 (FP64 work
+// about 2.5; the rest is the chain: a cluster barrier behind remote stores is
+// 1,650 clocks, each butterfly 500).  128 threads take 2.60 ms at n = 336, 256
+// 2.21, 512 2.35.
 template <int CS>
 __global__ void __launch_bounds__(kTriThreads)
 tridiag_kernel(int n, const double* __restrict__ A, int64_t lda, double* __restrict__ d, double* __restrict__ e,
                double* __restrict__ tau, double* __restrict__ V) {
+  static_assert(CS <= kMaxCluster, "slots");
   cg::cluster_group cl = cg::this_cluster();
   const int rank = CS > 1 ? (int)cl.block_rank() : 0;
   extern __shared__ double smem_d[];
   const int R = (n + CS - 1) / CS;
   double* Al = smem_d;
   double* vb = Al + (size_t)R * n;
-  double* pb = vb + 2 * n;
-  double* slots = pb + 2 * n;
-  double* red = slots + 64;
-  double* sc = red + 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  double* ub = vb + 2 * n;
+  double* slots = ub + 2 * n;
+  double* red = slots + 2 * kMaxCluster * kTriWarps;
+  double* sc = red + kTriWarps;  // 0: K, 1: w_j, 2: μ (μ + |α|), 3: τ
+  constexpr int kSlots = CS * kTriWarps, kPer = (kRitzMaxN + kTriThreads - 1) / kTriThreads;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int t = threadIdx.x; t < R * n; t += blockDim.x) {
     const int li = t / n, c = t % n;
     const int i = li * CS + rank;
     Al[t] = i < n ? A[(int64_t)i * lda + c] : 0.0;
   }
   if (CS > 1) cl.sync(); else __syncthreads();
-  for (int j = 0; j + 2 < n; ++j) {
-    const int par = j & 1;
-    double* v = vb + par * n;
-    double* p = pb + par * n;
-    double* wv = pb + (par ^ 1) * n;
-    double* sl = slots + par * 32;
-    if (rank == j % CS) {
-      // reflector of column j (= row j) below the diagonal, LAPACK dlarfg style
-      const double* row = Al + (size_t)(j / CS) * n;
-      double s = 0.0;
-      for (int k = j + 2 + threadIdx.x; k < n; k += blockDim.x) s = fma(row[k], row[k], s);
-      s = warp_sum_d(s);
-      if (lane == 0) red[warp] = s;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double sigma = 0.0;
-        for (int w = 0; w < nwarps; ++w) sigma += red[w];
-        const double alpha = row[j + 1];
-        double tj = 0.0, beta = alpha, scale = 0.0;
-        if (sigma > 0.0) {
-          const double mu = sqrt(fma(alpha, alpha, sigma));
-          beta = alpha <= 0.0 ? mu : -mu;
-          // τ = (β - α)/β and 1/(α - β) from one reciprocal
-          const double am = alpha - beta;
-          const double inv = 1.0 / (beta * am);
-          tj = -am * am * inv;
-          scale = beta * inv;
+  // steps 0 .. n-3 make reflectors; step n-2 only finishes the last 2 x 2 block
+  for (int j = 0; j + 1 < n; ++j) {
+    double* v = vb + (j & 1) * n;
+    const double* vp = vb + ((j & 1) ^ 1) * n;
+    double* w = ub + ((j & 1) ^ 1) * n;  // u of step j - 1, then its w
+    double* un = ub + (j & 1) * n;
+    const double* row_j = (CS > 1 ? cl.map_shared_rank(Al, j % CS) : Al) + (size_t)(j / CS) * n;
+    double rr[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int k = j + (int)threadIdx.x + q * kTriThreads;
+      rr[q] = k < n ? row_j[k] : 0.0;
+    }
+    if (j > 0) {
+      if (warp == 0) {
+        const double* sl = slots + ((j & 1) ^ 1) * (kMaxCluster * kTriWarps);
+        double x = 0.0;
+        for (int q = lane; q < kSlots; q += 32) x += sl[q];
+        x = warp_sum_d(x);
+        if (lane == 0) {
+          const double tp = sc[3], K = -0.5 * tp * (tp * x);
+          sc[0] = K;
+          sc[1] = fma(tp, w[j], K * vp[j]);
         }
-        sc[0] = tj;
-        sc[1] = scale;
-        sl[16] = tj;
-        d[j] = row[j];
-        e[j] = beta;
-        tau[j] = tj;
       }
       __syncthreads();
-      const double scale = sc[1];
-      for (int k = j + 1 + threadIdx.x; k < n; k += blockDim.x) {
-        const double vk = k == j + 1 ? 1.0 : row[k] * scale;
-        v[k] = vk;
-        V[(int64_t)j * n + k] = vk;
-      }
-      __syncthreads();
-      if (CS > 1) {
-        for (int r = 0; r < CS; ++r) {
-          if (r == rank) continue;
-          double* rv = cl.map_shared_rank(v, r);
-          for (int k = j + 1 + threadIdx.x; k < n; k += blockDim.x) rv[k] = v[k];
-          if (threadIdx.x == 0) cl.map_shared_rank(sl, r)[16] = sc[0];
+      const double tp = sc[3], K = sc[0], wj = sc[1], vj = vp[j];
+#pragma unroll
+      for (int q = 0; q < kPer; ++q) {
+        const int k = j + (int)threadIdx.x + q * kTriThreads;
+        if (k < n) {
+          const double wk = fma(tp, w[k], K * vp[k]);
+          w[k] = wk;
+          rr[q] = fma(-vj, wk, fma(-wj, vp[k], rr[q]));
         }
       }
     }
-    if (CS > 1) cl.sync(); else __syncthreads();
-    // p_i = τ Σ_k A[i][k] v_k over the trailing rows this CTA owns (warp per row)
-    const double tj = sl[16];
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int k = j + (int)threadIdx.x + q * kTriThreads;
+      if (k < n) {
+        v[k] = rr[q];
+        if (k >= j + 2) s = fma(rr[q], rr[q], s);
+      }
+    }
+    if (j + warp * 32 < n) s = warp_sum_d(s);  // a warp past the row's end has nothing to add
+    if (lane == 0) red[warp] = s;
+    __syncthreads();
+    if (j + 2 == n) break;
+    if (warp == 0) {
+      double sigma = lane < kTriWarps ? red[lane] : 0.0;
+#pragma unroll
+      for (int o = kTriWarps / 2; o; o >>= 1) sigma += __shfl_xor_sync(0xffffffffu, sigma, o);
+      if (lane == 0) {
+        const double alpha = v[j + 1];
+        double beta = alpha, den = 0.0;
+        if (sigma > 0.0) {
+          // x rsqrt(x): 350 + 64 clocks of this chain, a square root 675
+          const double x = fma(alpha, alpha, sigma), mu = x * rsqrt(x);
+          beta = alpha <= 0.0 ? mu : -mu;
+          den = mu * (mu + fabs(alpha));
+          v[j + 1] = alpha - beta;
+        }
+        sc[2] = den;
+        if (rank == j % CS) {
+          d[j] = v[j];
+          e[j] = beta;
+        }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == kTriThreads - 1) {  // the last warp has the fewest rows
+      const double den = sc[2], tj = den > 0.0 ? 1.0 / den : 0.0;
+      sc[3] = tj;
+      if (rank == j % CS) tau[j] = tj;
+    }
+    if (rank == (j + 1) % CS)  // not the CTA with the most rows left
+      for (int k = j + 1 + (int)threadIdx.x; k < n; k += kTriThreads) V[(int64_t)j * n + k] = v[k];
+    // owned trailing rows: A <- A - v_{j-1} wᵀ - w v_{j-1}ᵀ, u_i = A_i v
     const int first = j + 1 - rank;
     const int li0 = first <= 0 ? 0 : (first + CS - 1) / CS;
     double sv = 0.0;
-    for (int li = li0 + warp; li < R; li += nwarps) {
-      const int i = li * CS + rank;
-      if (i >= n) break;
-      const double* row = Al + (size_t)li * n;
-      double acc = 0.0;
-      for (int k = j + 1 + lane; k < n; k += 32) acc = fma(row[k], v[k], acc);
-      acc = warp_sum_d(acc) * tj;
-      sv = fma(acc, v[i], sv);
-      if (lane < CS) (CS > 1 ? cl.map_shared_rank(p, lane) : p)[i] = acc;
-    }
-    if (lane == 0) red[warp] = sv;
-    __syncthreads();
-    if (threadIdx.x < CS) {
-      double s2 = 0.0;
-      for (int w = 0; w < nwarps; ++w) s2 += red[w];
-      (CS > 1 ? cl.map_shared_rank(sl, (int)threadIdx.x) : sl)[rank] = s2;
-    }
-    if (CS > 1) cl.sync(); else __syncthreads();
-    // K = -τ/2 pᵀv (one warp), w = p + K v (once), A <- A - v wᵀ - w vᵀ on
-    // the owned trailing rows
-    if (warp == 0) {
-      const double x = warp_sum_d(lane < CS ? sl[lane] : 0.0);
-      if (lane == 0) sc[3] = -0.5 * tj * x;
-    }
-    __syncthreads();
-    const double K = sc[3];
-    for (int k = j + 1 + threadIdx.x; k < n; k += blockDim.x) wv[k] = fma(K, v[k], p[k]);
-    __syncthreads();
-    for (int li = li0 + warp; li < R; li += nwarps) {
+    for (int li = li0 + warp; li < R; li += kTriWarps) {
       const int i = li * CS + rank;
       if (i >= n) break;
       double* row = Al + (size_t)li * n;
-      const double vi = v[i], wi = wv[i];
-      for (int k = j + 1 + lane; k < n; k += 32) row[k] = fma(-vi, wv[k], fma(-wi, v[k], row[k]));
+      double acc = 0.0;
+      if (j > 0) {
+        const double vi = vp[i], wi = w[i];
+        for (int k = j + 1 + lane; k < n; k += 32) {
+          const double x = fma(-vi, w[k], fma(-wi, vp[k], row[k]));
+          row[k] = x;
+          acc = fma(x, v[k], acc);
+        }
+      } else {
+        for (int k = 1 + lane; k < n; k += 32) acc = fma(row[k], v[k], acc);
+      }
+      acc = warp_sum_d(acc);
+      sv = fma(acc, v[i], sv);
+      if (lane < CS) (CS > 1 ? cl.map_shared_rank(un, lane) : un)[i] = acc;
     }
-    __syncthreads();
+    if (lane < CS)
+      (CS > 1 ? cl.map_shared_rank(slots, lane) : slots)[(j & 1) * (kMaxCluster * kTriWarps) + rank * kTriWarps + warp] =
+          sv;
+    if (CS > 1) cl.sync(); else __syncthreads();
   }
-  // the last 2 x 2 block
-  if (threadIdx.x == 0) {
-    if (n >= 2 && rank == (n - 2) % CS) {
-      const double* row = Al + (size_t)((n - 2) / CS) * n;
-      d[n - 2] = row[n - 2];
-      e[n - 2] = row[n - 1];
+  // the last 2 x 2 block: row n-2 is in v of step n-2; the last diagonal
+  // element still lacks the last reflector's update
+  if (rank == 0 && threadIdx.x == 0) {
+    const double* row = (CS > 1 ? cl.map_shared_rank(Al, (n - 1) % CS) : Al) + (size_t)((n - 1) / CS) * n;
+    double x = row[n - 1];
+    if (n >= 2) {
+      const double* v = vb + ((n - 2) & 1) * n;
+      d[n - 2] = v[n - 2];
+      e[n - 2] = v[n - 1];
       tau[n - 2] = 0.0;
+      if (n >= 3) {
+        const double vl = vb[((n - 3) & 1) * n + n - 1], wl = ub[((n - 3) & 1) * n + n - 1];
+        x = fma(-vl, wl, fma(-wl, vl, x));
+      }
     }
-    if (rank == (n - 1) % CS) {
-      d[n - 1] = Al[(size_t)((n - 1) / CS) * n + n - 1];
-      tau[n - 1] = 0.0;
-    }
+    d[n - 1] = x;
+    tau[n - 1] = 0.0;
   }
   if (CS > 1) cl.sync();
 }
@@ -244,45 +279,59 @@ __device__ TriBounds tri_bounds_warp(int n, const double* __restrict__ d, const 
 // value of the sign opposite to its predecessor, which counts it as
 // negative, as the ratio form's pivot floor does.  Signs and exponents are
 // read as integers, off the FP64 pipe.
+// The common step is three FP64 operations and a range test on the high words;
+// the zero and rescaling cases, in which the whole warp takes part, are behind
+// one warp-uniform branch: as two conditions per lane they were compiled to
+// FP64 selects in every step, 695 clocks a step against 280 (1,280 -> 520 us
+// for 288 values of a 336 x 336 matrix).
 __device__ __forceinline__ int sturm_count(int n, const double* __restrict__ d, const double* __restrict__ e2,
                                            double x) {
-  constexpr long long kSign = (long long)0x8000000000000000ull;
+  constexpr unsigned kLow = (1023u - 400u) << 20, kHigh = (1023u + 401u) << 20;
   double pm = 1.0;
   double p = d[0] - x;
   if (p == 0.0) p = -DBL_MIN;
-  int c = p < 0.0;
+  unsigned hp = (unsigned)__double2hiint(p);
+  int c = (int)(hp >> 31);
   for (int i = 1; i < n; ++i) {
     double pn = fma(-e2[i - 1], pm, (d[i] - x) * p);
-    long long bn = __double_as_longlong(pn);
-    const long long bp = __double_as_longlong(p);
-    if ((bn & ~kSign) == 0) {  // zero minor: opposite sign to p, 2^-600 of the pair's scale (a normal number)
-      const double mag = fmax(fabs(p), fabs(pm)) * 0x1p-600;
-      pn = bp < 0 ? mag : -mag;
-      bn = __double_as_longlong(pn);
-    }
-    c += (int)(((unsigned long long)(bn ^ bp)) >> 63);
-    pm = p;
-    p = pn;
-    const int ex = (int)((bn >> 52) & 0x7ff), ey = (int)((bp >> 52) & 0x7ff);
-    const int emax = ex > ey ? ex : ey;
-    if (emax > 1023 + 400 || emax < 1023 - 400) {
-      // multiply both by 2^(1023 - emax), built from its bits
-      const double sc = __longlong_as_double((long long)(2046 - emax) << 52);
-      p *= sc;
-      pm *= sc;
+    unsigned hn = (unsigned)__double2hiint(pn);
+    // in range: the larger exponent of the pair within 2^±400 and the new
+    // minor a normal number
+    const unsigned an = hn & 0x7fffffffu, ap = hp & 0x7fffffffu, big = an > ap ? an : ap;
+    if (__any_sync(0xffffffffu, big - kLow >= kHigh - kLow || an < 0x00100000u)) {
+      if (pn == 0.0) {  // opposite sign to p, 2^-600 of the pair's scale (a normal number)
+        const double mag = fmax(fabs(p), fabs(pm)) * 0x1p-600;
+        pn = p < 0.0 ? mag : -mag;
+      }
+      c += (int)(((unsigned)__double2hiint(pn) ^ hp) >> 31);
+      pm = p;
+      p = pn;
+      const int ex = (__double2hiint(p) >> 20) & 0x7ff, ey = (__double2hiint(pm) >> 20) & 0x7ff;
+      const int emax = ex > ey ? ex : ey;
+      if (emax > 1023 + 400 || emax < 1023 - 400) {
+        // multiply both by 2^(1023 - emax), built from its bits
+        const double sc = __longlong_as_double((long long)(2046 - emax) << 52);
+        p *= sc;
+        pm *= sc;
+      }
+      hp = (unsigned)__double2hiint(p);
+    } else {
+      c += (int)((hn ^ hp) >> 31);
+      pm = p;
+      p = pn;
+      hp = hn;
     }
   }
   return c;
 }
 
-// lam[w] = eigenvalue of ascending rank ranks[w].  A group of kBisLanes lanes
-// per wanted value evaluates kBisLanes shifts per round (multisection into
-// kBisLanes + 1 parts).  A warp's FP64 instructions run one after another on
-// its sub-partition's FP64 unit whatever the number of active lanes, so the
-// time is rounds x steps x FP64 operations per step of one warp, with one
-// warp per sub-partition (two-warp blocks).  d and e² are staged in shared
-// memory.
-constexpr int kBisLanes = 32;
+// lam[w] = eigenvalue of ascending rank ranks[w].  A warp per wanted value
+// evaluates 32 shifts per round (multisection into 33 parts).  A warp's FP64
+// instructions run one after another on its sub-partition's FP64 unit, 64
+// clocks each whatever the number of active lanes, so the time is rounds x
+// steps x FP64 operations per step of one warp, with one warp per
+// sub-partition (two-warp blocks); two shifts per lane take twice as long per
+// round and save two rounds in eleven.  d and e² are staged in shared memory.
 constexpr int kBisThreads = 64;
 __global__ void __launch_bounds__(kBisThreads)
 bisect_kernel(int n, const double* __restrict__ d, const double* __restrict__ e, const int* __restrict__ ranks, int nw,
@@ -307,33 +356,24 @@ bisect_kernel(int n, const double* __restrict__ d, const double* __restrict__ e,
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  constexpr int GPW = 32 / kBisLanes;
-  const int g = lane / kBisLanes, gl = lane % kBisLanes;
-  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * GPW + g;
-  if ((int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * GPW >= nw) return;  // whole warp idle
-  const bool active = w < nw;
-  const int r = active ? ranks[w] : 0;
-  constexpr double kStep = 1.0 / (kBisLanes + 1);
+  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  if (w >= nw) return;
+  const int r = ranks[w];
+  constexpr double kStep = 1.0 / 33.0;
   const double tnorm = bs.tnorm * sc;
   double lo = bs.lo * sc, hi = bs.hi * sc;
-  const unsigned gmask = kBisLanes == 32 ? 0xffffffffu : ((1u << (kBisLanes % 32)) - 1u) << (g * kBisLanes);
   for (int it = 0; it < 64; ++it) {
     const double width = hi - lo;
-    const bool done = !active || width <= 0.0 ||
-                      width <= fmax(DBL_EPSILON * tnorm, 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)));
-    if (__all_sync(0xffffffffu, done)) break;
-    int c = 0;
-    if (!done) c = sturm_count(n, ds, e2s, lo + width * ((gl + 1) * kStep));
-    const unsigned above = (__ballot_sync(0xffffffffu, c > r) & gmask) >> ((g * kBisLanes) % 32);
-    if (!done) {
-      const int l = above ? __ffs(above) - 1 : kBisLanes;
-      const double nlo = l == 0 ? lo : lo + width * (l * kStep);
-      const double nhi = l == kBisLanes ? hi : lo + width * ((l + 1) * kStep);
-      lo = nlo;
-      hi = nhi;
-    }
+    if (width <= 0.0 || width <= fmax(DBL_EPSILON * tnorm, 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)))) break;
+    const int c = sturm_count(n, ds, e2s, lo + width * ((lane + 1) * kStep));
+    const unsigned above = __ballot_sync(0xffffffffu, c > r);
+    const int l = above ? __ffs(above) - 1 : 32;
+    const double nlo = l == 0 ? lo : lo + width * (l * kStep);
+    const double nhi = l == 32 ? hi : lo + width * ((l + 1) * kStep);
+    lo = nlo;
+    hi = nhi;
   }
-  if (active && gl == 0) lam[w] = 0.5 * (lo + hi) * isc;
+  if (lane == 0) lam[w] = 0.5 * (lo + hi) * isc;
 }
 
 __device__ __forceinline__ double hash_unit(uint64_t a, uint64_t b) {
@@ -482,14 +522,17 @@ __global__ void invit_kernel(int n, const double* __restrict__ d, const double* 
   }
 }
 
-// G (lower triangle) = Zt Ztᵀ over the nw rows of length n; one warp per entry
-__global__ void gram_rows_kernel(int nw, int n, const double* __restrict__ Zt, double* __restrict__ G) {
+// E = Zt Ztᵀ - I over the nw rows of length n, both triangles; one warp per
+// entry of the lower one.  *wide counts the entries too large for the
+// iteration below: with every |E_ij| <= 1 / (4 nw), ‖E‖ <= 1/4.
+__global__ void gram_rows_kernel(int nw, int n, const double* __restrict__ Zt, double* __restrict__ E,
+                                 int* __restrict__ wide) {
   const int lane = threadIdx.x & 31;
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t tot = (int64_t)nw * (nw + 1) / 2;
   if (w >= tot) return;
   // w -> (i, j), j <= i
-  int i = (int)((sqrt(8.0 * (double)w + 1.0) - 1.0) * 0.5);
+  int i = (int)((sqrtf(8.0f * (float)w + 1.0f) - 1.0f) * 0.5f);
   while ((int64_t)i * (i + 1) / 2 > w) --i;
   while ((int64_t)(i + 1) * (i + 2) / 2 <= w) ++i;
   const int j = (int)(w - (int64_t)i * (i + 1) / 2);
@@ -498,14 +541,53 @@ __global__ void gram_rows_kernel(int nw, int n, const double* __restrict__ Zt, d
   double s = 0.0;
   for (int c = lane; c < n; c += 32) s = fma(a[c], b[c], s);
   s = warp_sum_d(s);
-  if (lane == 0) G[(size_t)i * nw + j] = s;
+  if (lane == 0) {
+    if (i == j) s -= 1.0;
+    E[(size_t)i * nw + j] = s;
+    E[(size_t)j * nw + i] = s;
+    if (wide && !(fabs(s) * (4.0 * nw) <= 1.0)) atomicAdd(wide, 1);
+  }
 }
 
-// Cholesky G = L Lᵀ in place (lower), then Zt <- L⁻¹ Zt (rows orthonormal).
-// One CTA; a non-positive pivot leaves Zt as it is.
-__global__ void __launch_bounds__(1024) orth_kernel(int nw, int n, double* __restrict__ G, double* __restrict__ Zt) {
+// out = Zt - E Zt / 2 (rows): one step of Björck and Bowie's iteration for
+// the closest orthonormal matrix (SIAM J. Numer. Anal. 8 (1971) 358), whose
+// error E becomes 3/4 E².  A warp holds 32 columns of kOrthRows rows, so a
+// load of Zt serves kOrthRows FMAs.  Nothing is done when *wide is set.
+constexpr int kOrthRows = 4;
+__global__ void __launch_bounds__(128)
+orth_step_kernel(int nw, int n, const double* __restrict__ E, const double* __restrict__ Zt,
+                 double* __restrict__ out, const int* __restrict__ wide) {
+  if (*wide) return;
+  const int c = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 32 + (threadIdx.x & 31);
+  if (c >= n) return;
+  const int i0 = blockIdx.y * kOrthRows;
+  double acc[kOrthRows];
+  const double* er[kOrthRows];
+#pragma unroll
+  for (int r = 0; r < kOrthRows; ++r) {
+    acc[r] = 0.0;
+    er[r] = E + (size_t)min(i0 + r, nw - 1) * nw;
+  }
+#pragma unroll 4
+  for (int q = 0; q < nw; ++q) {
+    const double z = Zt[(size_t)q * n + c];
+#pragma unroll
+    for (int r = 0; r < kOrthRows; ++r) acc[r] = fma(er[r][q], z, acc[r]);
+  }
+#pragma unroll
+  for (int r = 0; r < kOrthRows; ++r)
+    if (i0 + r < nw) out[(size_t)(i0 + r) * n + c] = fma(-0.5, acc[r], Zt[(size_t)(i0 + r) * n + c]);
+}
+
+// For vectors too far from orthonormal for the iteration (*wide set; nothing
+// is done otherwise): G = E + I = L Lᵀ in place (lower), then Zt <- L⁻¹ Zt
+// (rows orthonormal).  One CTA; a non-positive pivot leaves Zt as it is.
+__global__ void __launch_bounds__(1024)
+orth_kernel(int nw, int n, double* __restrict__ G, double* __restrict__ Zt, const int* __restrict__ wide) {
+  if (!*wide) return;
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
+  for (int i = threadIdx.x; i < nw; i += blockDim.x) G[(size_t)i * nw + i] += 1.0;
   __syncthreads();
   for (int j = 0; j < nw; ++j) {
     if (threadIdx.x == 0) {
@@ -536,28 +618,117 @@ __global__ void __launch_bounds__(1024) orth_kernel(int nw, int n, double* __res
   }
 }
 
-// Zt rows <- Q Zt rows, Q = H_0 H_1 ... H_{n-3}; one warp per vector
-__global__ void backtr_kernel(int n, const double* __restrict__ V, const double* __restrict__ tau, int nw,
-                              double* __restrict__ Zt) {
-  extern __shared__ double zsh[];
-  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  if (w >= nw) return;
-  double* z = zsh + (size_t)wl * n;
-  double* g = Zt + (size_t)w * n;
-  for (int i = lane; i < n; i += 32) z[i] = g[i];
+// Reflectors are applied kWy at a time: H_j H_{j+1} ... H_{j+kWy-1} =
+// I - W T Wᵀ with the reflectors as the columns of W and T upper triangular
+// (the compact WY form; Schreiber and Van Loan, SIAM J. Sci. Stat. Comput. 10
+// (1989) 53): T_cc = τ_c, T_{0..c-1,c} = -τ_c T_{0..c-1,0..c-1} W_{0..c-1}ᵀ w_c.
+// One warp per block of reflectors; row j of V holds reflector j from j + 1 on.
+constexpr int kWy = 8;
+__global__ void __launch_bounds__(32)
+wy_kernel(int n, const double* __restrict__ V, const double* __restrict__ tau, double* __restrict__ T) {
+  const int j0 = blockIdx.x * kWy, nr = n - 2, lane = threadIdx.x;
+  __shared__ double g[kWy][kWy], t[kWy][kWy];
+  double acc[kWy * kWy / 2 + kWy];  // packed pairs a < c
+#pragma unroll
+  for (int x = 0; x < kWy * (kWy - 1) / 2; ++x) acc[x] = 0.0;
+  for (int k = j0 + 1 + lane; k < n; k += 32) {
+    double v[kWy];
+#pragma unroll
+    for (int c = 0; c < kWy; ++c) v[c] = j0 + c < nr && k > j0 + c ? V[(int64_t)(j0 + c) * n + k] : 0.0;
+    int x = 0;
+#pragma unroll
+    for (int a = 0; a < kWy; ++a)
+#pragma unroll
+      for (int c = a + 1; c < kWy; ++c) acc[x] = fma(v[a], v[c], acc[x]), ++x;
+  }
+  int x = 0;
+#pragma unroll
+  for (int a = 0; a < kWy; ++a)
+#pragma unroll
+    for (int c = a + 1; c < kWy; ++c) {
+      const double s = warp_sum_d(acc[x++]);
+      if (lane == 0) g[a][c] = s;
+    }
+  for (int q = lane; q < kWy * kWy; q += 32) t[q / kWy][q % kWy] = 0.0;
   __syncwarp();
-  for (int j = n - 3; j >= 0; --j) {
-    const double tj = tau[j];
-    if (tj == 0.0) continue;
-    const double* vj = V + (size_t)j * n;
+  for (int c = 0; c < kWy; ++c) {
+    const double tc = j0 + c < nr ? tau[j0 + c] : 0.0;
     double s = 0.0;
-    for (int k = j + 1 + lane; k < n; k += 32) s = fma(vj[k], z[k], s);
-    s = warp_sum_d(s) * tj;
-    for (int k = j + 1 + lane; k < n; k += 32) z[k] = fma(-s, vj[k], z[k]);
+    if (lane < c)
+      for (int q = lane; q < c; ++q) s = fma(t[lane][q], g[q][c], s);
+    __syncwarp();
+    if (lane < c) t[lane][c] = -tc * s;
+    if (lane == c) t[c][c] = tc;
     __syncwarp();
   }
-  for (int i = lane; i < n; i += 32) g[i] = z[i];
+  for (int q = lane; q < kWy * kWy; q += 32) T[(int64_t)blockIdx.x * kWy * kWy + q] = t[q / kWy][q % kWy];
+}
+
+// Zt rows <- Q Zt rows, Q = H_0 H_1 ... H_{n-3}; one CTA per vector, its
+// elements in registers.  A block of reflectors costs eight dot products side
+// by side (one transpose butterfly), eight FMAs for T and the update, instead
+// of eight dependent dot products of five additions each by one warp: 586 ->
+// 300 us (and 22 us for T) for 288 vectors at n = 336.
+constexpr int kBackThreads = 128;
+__global__ void __launch_bounds__(kBackThreads)
+backtr_kernel(int n, const double* __restrict__ V, const double* __restrict__ T, double* __restrict__ Zt) {
+  constexpr int kPer = (kRitzMaxN + kBackThreads - 1) / kBackThreads, kWarps = kBackThreads / 32;
+  __shared__ double ys[2][kWarps][kWy];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nr = n - 2;
+  double* g = Zt + (size_t)blockIdx.x * n;
+  double z[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int k = (int)threadIdx.x + q * kBackThreads;
+    z[q] = k < n ? g[k] : 0.0;
+  }
+  for (int b = (nr + kWy - 1) / kWy - 1; b >= 0; --b) {
+    const int j0 = b * kWy;
+    const double* Tb = T + (int64_t)b * kWy * kWy;
+    double v[kPer][kWy], y[kWy];
+#pragma unroll
+    for (int c = 0; c < kWy; ++c) y[c] = 0.0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int k = (int)threadIdx.x + q * kBackThreads;
+#pragma unroll
+      for (int c = 0; c < kWy; ++c)
+        v[q][c] = k < n && j0 + c < nr && k > j0 + c ? V[(int64_t)(j0 + c) * n + k] : 0.0;
+    }
+    // lane c's row of T, in flight beside the reflectors
+    double tr[kWy];
+#pragma unroll
+    for (int c = 0; c < kWy; ++c) tr[c] = Tb[(lane % kWy) * kWy + c];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      if (warp * 32 + q * kBackThreads < n && warp * 32 + q * kBackThreads + 31 > j0) {
+#pragma unroll
+        for (int c = 0; c < kWy; ++c) y[c] = fma(v[q][c], z[q], y[c]);
+      }
+    }
+    warp_colsum<double, kWy>(y, lane);
+    if (lane % (32 / kWy) == 0) ys[b & 1][warp][lane / (32 / kWy)] = y[0];
+    __syncthreads();
+    // lane: y_c of c = lane mod 8 summed over the warps, then (T y)_c
+    double yc = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) yc += ys[b & 1][w][lane % kWy];
+    double t = 0.0;
+#pragma unroll
+    for (int c = 0; c < kWy; ++c) t = fma(tr[c], __shfl_sync(0xffffffffu, yc, c), t);
+#pragma unroll
+    for (int c = 0; c < kWy; ++c) {
+      const double tc = -__shfl_sync(0xffffffffu, t, c);
+#pragma unroll
+      for (int q = 0; q < kPer; ++q)
+        if (warp * 32 + q * kBackThreads < n && warp * 32 + q * kBackThreads + 31 > j0) z[q] = fma(tc, v[q][c], z[q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int k = (int)threadIdx.x + q * kBackThreads;
+    if (k < n) g[k] = z[q];
+  }
 }
 
 __global__ void ranks_kernel(int n, int p, int q, int* __restrict__ ranks) {
@@ -641,7 +812,7 @@ RitzLayout ritz_layout(char* base, int n, int nw) {
   const int64_t od = take(8 * (int64_t)n), oe = take(8 * (int64_t)n), ot = take(8 * (int64_t)n),
                 oV = take(8 * (int64_t)n * n), orr = take(4 * (int64_t)n), ol = take(8 * (int64_t)n),
                 oz = take(8 * (int64_t)n * nw), olu = take(32 * (int64_t)n * nw), op = take((int64_t)n * nw),
-                oG = take(8 * (int64_t)nw * nw);
+                oG = take(8 * (int64_t)nw * nw), oT = take(8 * kWy * ((int64_t)n + kWy)), ow = take(4);
   if (base) {
     L.d = (double*)(base + od);
     L.e = (double*)(base + oe);
@@ -653,6 +824,8 @@ RitzLayout ritz_layout(char* base, int n, int nw) {
     L.lu = (double*)(base + olu);
     L.piv = (unsigned char*)(base + op);
     L.G = (double*)(base + oG);
+    L.T = (double*)(base + oT);
+    L.wide = (int*)(base + ow);
   }
   L.bytes = o;
   return L;
@@ -676,8 +849,7 @@ int ritz_values(int n, const double* A, int64_t lda, int p, int q, const RitzLay
   if (err) return err;
   ranks_kernel<<<grid_for(cnt, 256), 256, 0, s>>>(n, p, q, L.ranks);
   SG_CHECK_LAUNCH();
-  bisect_kernel<<<grid_for((int64_t)cnt * kBisLanes, kBisThreads), kBisThreads, 0, s>>>(n, L.d, L.e, L.ranks, cnt,
-                                                                                         L.lam);
+  bisect_kernel<<<grid_for((int64_t)cnt * 32, kBisThreads), kBisThreads, 0, s>>>(n, L.d, L.e, L.ranks, cnt, L.lam);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -689,16 +861,28 @@ int ritz_vectors(int n, const RitzLayout& L, const int* sel, int nsel, cudaStrea
   invit_kernel<<<grid_for((int64_t)nsel * 32, 128), 128, 0, s>>>(n, L.d, L.e, L.ranks, L.lam, sel, nsel, L.Zt, L.lu,
                                                                   L.piv);
   SG_CHECK_LAUNCH();
-  constexpr int wpb = 4;
-  const size_t sm = (size_t)wpb * n * sizeof(double);
-  static_assert(wpb * kRitzMaxN * sizeof(double) <= 48 * 1024, "back-transformation fits default shared memory");
-  backtr_kernel<<<(nsel + wpb - 1) / wpb, 32 * wpb, sm, s>>>(n, L.V, L.tau, nsel, L.Zt);
-  SG_CHECK_LAUNCH();
-  if (nsel > 1) {
-    const int64_t pairs = (int64_t)nsel * (nsel + 1) / 2;
-    gram_rows_kernel<<<grid_for(pairs * 32, 256), 256, 0, s>>>(nsel, n, L.Zt, L.G);
+  if (n > 2) {
+    wy_kernel<<<(n - 2 + kWy - 1) / kWy, 32, 0, s>>>(n, L.V, L.tau, L.T);
     SG_CHECK_LAUNCH();
-    orth_kernel<<<1, 1024, 0, s>>>(nsel, n, L.G, L.Zt);
+    backtr_kernel<<<nsel, kBackThreads, 0, s>>>(n, L.V, L.T, L.Zt);
+    SG_CHECK_LAUNCH();
+  }
+  if (nsel > 1) {
+    // two steps of the iteration through the inverse iteration's scratch and
+    // back; the second finds ‖E‖ <= 3/64 at worst and about 1e-14 as a rule
+    double* Z2 = L.lu;
+    const int64_t pairs = (int64_t)nsel * (nsel + 1) / 2;
+    const dim3 grid((n + 127) / 128, (nsel + kOrthRows - 1) / kOrthRows);
+    if (cudaMemsetAsync(L.wide, 0, sizeof(int), s) != cudaSuccess) return SG_ERR_CUDA;
+    gram_rows_kernel<<<grid_for(pairs * 32, 256), 256, 0, s>>>(nsel, n, L.Zt, L.G, L.wide);
+    SG_CHECK_LAUNCH();
+    orth_kernel<<<1, 1024, 0, s>>>(nsel, n, L.G, L.Zt, L.wide);
+    SG_CHECK_LAUNCH();
+    orth_step_kernel<<<grid, 128, 0, s>>>(nsel, n, L.G, L.Zt, Z2, L.wide);
+    SG_CHECK_LAUNCH();
+    gram_rows_kernel<<<grid_for(pairs * 32, 256), 256, 0, s>>>(nsel, n, Z2, L.G, nullptr);
+    SG_CHECK_LAUNCH();
+    orth_step_kernel<<<grid, 128, 0, s>>>(nsel, n, L.G, Z2, L.Zt, L.wide);
     SG_CHECK_LAUNCH();
   }
   return SG_OK;
