@@ -18,20 +18,26 @@
 // a NaN sends the whole call through FP64 additions (uniform branch), so
 // non-finite values propagate as before.
 //
-// Layout: CTAs of 8 warps own R consecutive rows.  A warp sums its rows one
-// by one, B/2 lanes per nonzero (16-byte gathers), and keeps each row's sum in
-// the lanes of one slot, so that one epilogue with all lanes busy (an idle
-// lane costs an FP64 slot too) scales 64/B rows.  Rows of more than kLong
-// nonzeros are summed by the whole CTA afterwards.  R is the largest size
-// that still gives every SM eight CTAs (short matrices take 4 rows a CTA).
-// Four CTAs per SM (64 registers) beat three by 3-10 % and five by more; two
-// index chunks in flight at 8 columns beat one (20 %) and four (30 %).
+// Layout: CTAs of 8 warps own R consecutive rows, and each warp an equal slice
+// of their nonzeros, wherever the row ends fall: a row that lies in several
+// slices is put together in shared memory at the end (a warp per row, with the
+// rows above 512 nonzeros shared by the CTA and a barrier for each, waited 21 %
+// of its time at barriers on rows of unequal length).  B/2 lanes take one
+// nonzero (16-byte gathers); a row's sum is folded over the warp and left in
+// shared memory, and one epilogue with all lanes busy (an idle lane costs an
+// FP64 slot too) scales all the CTA's rows, a thread to two columns of one.
+// Column indices are loaded one step ahead of the gathers, and a step's unused
+// lanes read a row of zeros (3-9 % faster than a test per gather).
+// Four CTAs per SM (64 registers) beat three by 1-40 % and five by more; two
+// index chunks in flight at 8 columns beat one (10-30 %) and four (twice).
 //
 // Measured, Xᵀ / X pass with the FP64 kernel's best variant in brackets:
-// 5,000 x 200,003, 2.1e7 nonzeros, 8 columns: 167 / 159 us (502 / 495); 2,000
-// x 50,000, 3.1e6, 8 columns: 39 / 40 us (95 / 88); 20,000 x 300,000, 8.3e7:
-// 4 columns 0.39 / 0.43 ms (0.97 / 0.74), 32 columns 1.39 / 1.85 ms (6.1 /
-// 5.9), where the 256-byte rows arrive at 15 / 11 TB/s.  The gathers bind now.
+// 5,000 x 200,003, 2.1e7 nonzeros, 8 columns: 140 / 125 us (502 / 495); 2,000
+// x 50,000, 3.1e6, 8 columns: 38 / 34 us (95 / 88); 20,000 x 300,000, 8.3e7:
+// 4 columns 0.34 / 0.33 ms (0.97 / 0.74), 32 columns 0.97 / 1.13 ms (6.1 /
+// 5.9), where the 256-byte rows arrive at 22 / 19 TB/s.  (A warp per short row
+// and a CTA per long one: 167 / 159, 39 / 40, 390 / 430, 1,390 / 1,850.)  The
+// L1's lookups bind now (about 75 % of its peak).
 #include "common.cuh"
 #include "internal.h"
 
@@ -40,7 +46,9 @@ namespace {
 
 constexpr int kFxThreads = 256;
 constexpr int kFxWarps = kFxThreads / 32;
-constexpr int kLong = 512;         // nonzeros above which a row is shared by the CTA's warps
+constexpr int kFxCtas = 4;       // CTAs per SM (64 registers)
+template <int B>
+constexpr int kFxMaxRows = kFxWarps * (64 / B);  // rows per CTA at most
 constexpr int kHeadBytes = 256;    // per-column maxima in front of the integers
 constexpr unsigned kNonFinite = 0x7ff00000u;
 
@@ -88,6 +96,7 @@ fx_quantize_kernel(int64_t nvec, const double2* __restrict__ in, const unsigned*
   const int c = 2 * (threadIdx.x % (B / 2));
   const unsigned ha = head[c], hb = head[c + 1];
   if (ha >= kNonFinite || hb >= kNonFinite) return;  // the sums are taken in FP64 then
+  if (blockIdx.x == 0 && threadIdx.x < B / 2) q[nvec + threadIdx.x] = make_ulonglong2(0, 0);  // read past a row's end
   const int sa = fx_shift(ha), sb = fx_shift(hb);
   for (int64_t i = blockIdx.x * (int64_t)kFxThreads + threadIdx.x; i < nvec; i += stride) {
     const double2 v = in[i];
@@ -140,42 +149,57 @@ struct Acc {
   }
 };
 
-// adds CH chunks of 32 nonzeros starting at k0 (entries at or past e are skipped)
-template <int B, int CH>
-__device__ __forceinline__ void fx_chunk(Acc<B>& acc, int64_t k0, int64_t e, const int32_t* __restrict__ idx,
-                                         const ulonglong2* __restrict__ q, int lane) {
+// column indices of the first CH chunks of 32 of n nonzeros; past them the row
+// of zeros behind the operand, which the gathers read without a test
+template <int CH>
+__device__ __forceinline__ void fx_load(int (&ci)[CH], const int32_t* __restrict__ p, int n, int zero, int lane) {
+#pragma unroll
+  for (int c = 0; c < CH; ++c) ci[c] = c * 32 + lane < n ? __ldg(p + c * 32 + lane) : zero;
+}
+
+// adds the rows named by the first N chunks of ci
+template <int B, int CH, int N>
+__device__ __forceinline__ void fx_add(Acc<B>& acc, const int (&ci)[CH], const ulonglong2* __restrict__ q, int lane) {
   constexpr int LPN = B / 2, NPS = 32 / LPN;
   constexpr int GB = LPN < 8 ? LPN : 8;  // gathers in flight per chunk
   const int sub = lane % LPN, slot = lane / LPN;
-  int ci[CH];
-#pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int64_t k = k0 + c * 32 + lane;
-    ci[c] = k < e ? __ldg(idx + k) : -1;
-  }
 #pragma unroll
   for (int j0 = 0; j0 < LPN; j0 += GB) {
-    ulonglong2 g[CH * GB];
+    ulonglong2 g[N * GB];
 #pragma unroll
-    for (int c = 0; c < CH; ++c)
+    for (int c = 0; c < N; ++c)
 #pragma unroll
       for (int j = 0; j < GB; ++j) {
-        const int col = __shfl_sync(0xffffffffu, ci[c], (j0 + j) * NPS + slot);
-        g[c * GB + j] = col >= 0 ? __ldg(q + (int64_t)col * LPN + sub) : make_ulonglong2(0, 0);
+        const unsigned col = (unsigned)__shfl_sync(0xffffffffu, ci[c], (j0 + j) * NPS + slot);
+        g[c * GB + j] = __ldg(q + (uint64_t)col * LPN + sub);
       }
 #pragma unroll
-    for (int t = 0; t < CH * GB; ++t) acc.add(g[t]);
+    for (int t = 0; t < N * GB; ++t) acc.add(g[t]);
   }
 }
 
-// chunks k0, k0 + step, ... of a row
 template <int B>
-__device__ __forceinline__ void fx_row(Acc<B>& acc, int64_t k0, int64_t e, int64_t step,
-                                       const int32_t* __restrict__ idx, const ulonglong2* __restrict__ q, int lane) {
-  constexpr int CH = B == 4 ? 4 : (B == 8 ? 2 : 1);
-  for (; k0 < e; k0 += step) {
-    if (CH == 1 || k0 + 32 < e) fx_chunk<B, CH>(acc, k0, e, idx, q, lane);
-    else fx_chunk<B, 1>(acc, k0, e, idx, q, lane);
+constexpr int kChunks = B == 4 ? 4 : (B == 8 ? 2 : 1);
+
+// n nonzeros of a row from p on; ci holds the indices of the first
+// chunks and receives those of the next nn nonzeros after the row (the warp's
+// next row).  Indices are loaded one step ahead, so a step waits for the
+// gathers alone.
+template <int B>
+__device__ __forceinline__ void fx_row(Acc<B>& acc, int (&ci)[kChunks<B>], const int32_t* __restrict__ p, int n,
+                                       int nn, int zero, const ulonglong2* __restrict__ q, int lane) {
+  constexpr int CH = kChunks<B>, STEP = 32 * CH;
+  while (n > 0) {
+    int next[CH];
+    const int adv = n < STEP ? n : STEP;
+    p += adv;
+    fx_load<CH>(next, p, n > STEP ? n - STEP : nn, zero, lane);
+    if (CH == 1 || n > 16 * CH) fx_add<B, CH, CH>(acc, ci, q, lane);
+    else if (CH == 4 && n > 32) fx_add<B, CH, CH == 4 ? 2 : 1>(acc, ci, q, lane);
+    else fx_add<B, CH, 1>(acc, ci, q, lane);
+#pragma unroll
+    for (int c = 0; c < CH; ++c) ci[c] = next[c];
+    n -= STEP;
   }
 }
 
@@ -198,31 +222,31 @@ __device__ __forceinline__ void fx_store(int64_t r, int sub, double a, double b,
 }
 
 template <int B, bool SHIFT>
-__global__ void __launch_bounds__(kFxThreads, 4)
-spmm_fx_kernel(int64_t rows, int R, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+__global__ void __launch_bounds__(kFxThreads, kFxCtas)
+spmm_fx_kernel(int64_t rows, int R, int zero, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                const double* __restrict__ in, const ulonglong2* __restrict__ q, const unsigned* __restrict__ head,
                double* __restrict__ out, const double* __restrict__ scale, const double* __restrict__ dshift,
                const double* __restrict__ y) {
   constexpr int LPN = B / 2, NPS = 32 / LPN;
-  constexpr int CH = B == 4 ? 4 : (B == 8 ? 2 : 1);
-  static_assert(NPS * kFxWarps <= kFxThreads, "one thread per row of the CTA");
-  __shared__ int64_t s_ptr[kFxWarps * NPS + 1];
-  __shared__ int s_long[kFxWarps * NPS];
-  __shared__ int s_nlong;
-  __shared__ unsigned s_part[2][kFxWarps][LPN][6];
+  constexpr int CH = kChunks<B>;
+  __shared__ int s_off[kFxMaxRows<B> + 2];  // row offsets in the CTA's nonzeros (below 2^31), the last one twice
+  __shared__ unsigned s_sum[6][kFxMaxRows<B> * LPN];  // of the rows, less the pieces in s_piece
+  __shared__ unsigned s_piece[6][kFxWarps * LPN];     // a warp's piece of the row that its slice ends inside of
+  __shared__ int s_tail[kFxWarps];                    // that row, or -1
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane % LPN, slot = lane / LPN;
   const int64_t r0 = blockIdx.x * (int64_t)R;
   const int nr = (int)(rows - r0 < R ? rows - r0 : R);
-  if (threadIdx.x == 0) s_nlong = 0;
-  if (threadIdx.x <= nr) s_ptr[threadIdx.x] = ptr[r0 + threadIdx.x];
+  const int64_t p0 = ptr[r0];
+  if (threadIdx.x <= nr + 1) s_off[threadIdx.x] = (int)(ptr[r0 + min((int)threadIdx.x, nr)] - p0);
+  idx += p0;
   const unsigned ha = head[2 * sub], hb = head[2 * sub + 1];
   const bool finite = __all_sync(0xffffffffu, ha < kNonFinite && hb < kNonFinite);  // the same in every warp
   __syncthreads();
   if (!finite) {  // FP64 additions, a warp per row
     for (int i = warp; i < nr; i += kFxWarps) {
       double2 acc = make_double2(0.0, 0.0);
-      for (int64_t k = s_ptr[i] + slot; k < s_ptr[i + 1]; k += NPS)
+      for (int k = s_off[i] + slot; k < s_off[i + 1]; k += NPS)
         V16<double>::add(acc, *reinterpret_cast<const double2*>(in + (int64_t)idx[k] * B + 2 * sub));
       __syncwarp();
 #pragma unroll
@@ -231,58 +255,60 @@ spmm_fx_kernel(int64_t rows, int R, const int64_t* __restrict__ ptr, const int32
     }
     return;
   }
-  const int sa = fx_shift(ha), sb = fx_shift(hb);
-  if (threadIdx.x < nr && s_ptr[threadIdx.x + 1] - s_ptr[threadIdx.x] > kLong)
-    s_long[atomicAdd(&s_nlong, 1)] = threadIdx.x;
-  // rows of this warp, one after the other; row i of the warp ends up in slot i
-  const int per = R < kFxWarps ? 1 : R / kFxWarps;  // <= NPS
-  Acc<B> mine;
-  mine.zero();
-  unsigned mylen = 0;
-  int myrow = -1;
-  for (int i = 0; i < per; ++i) {
-    const int t = warp * per + i;
-    if (t >= nr) break;
-    const int64_t s = s_ptr[t], e = s_ptr[t + 1];
-    if (e - s > kLong) continue;
+  // this warp's slice [sl, sh) of the CTA's nonzeros; it finishes the rows
+  // that end in (sl, sh] (warp 0 also the empty ones in front)
+  const int total = s_off[nr], per = (total / kFxWarps + 32) / 32 * 32;
+  const int sl = (int)min((int64_t)warp * per, (int64_t)total), sh = min((int64_t)sl + per, (int64_t)total);
+  int t = 0;
+  if (warp > 0)
+    for (int i = 0; i < nr; i += 32) t += __popc(__ballot_sync(0xffffffffu, i + lane < nr && s_off[i + lane + 1] <= sl));
+  const int32_t* p = idx + sl;
+  int ci[CH], e = s_off[min(t, nr) + 1], n = t < nr ? min(e, sh) - sl : 0;
+  int tail = -1;
+  fx_load<CH>(ci, p, n, zero, lane);
+  for (; t < nr; ++t) {
+    const bool ends = e <= sh;
+    if (!ends && n == 0) break;
+    const int e2 = s_off[t + 2], nn = min(e2, sh) - min(e, sh);
     Acc<B> acc;
     acc.zero();
-    fx_row<B>(acc, s, e, 32 * CH, idx, q, lane);
-    acc.fold();
-    if (slot == i) {
-      mine = acc;
-      mylen = (unsigned)(e - s);
-      myrow = t;
-    }
-  }
-  if (myrow >= 0)
-    fx_store<B, SHIFT>(r0 + myrow, sub, mine.a.value(mylen, sa), mine.b.value(mylen, sb), out, scale, dshift, y);
-  __syncthreads();
-  // long rows, by all warps; one barrier a row (the partial sums alternate between two buffers)
-  const int nl = s_nlong;
-  for (int l = 0; l < nl; ++l) {
-    const int t = s_long[l];
-    const int64_t s = s_ptr[t], e = s_ptr[t + 1];
-    Acc<B> acc;
-    acc.zero();
-    fx_row<B>(acc, s + (int64_t)warp * 32 * CH, e, (int64_t)kFxWarps * 32 * CH, idx, q, lane);
+    if (n == 0) fx_load<CH>(ci, p, nn, zero, lane);
+    else fx_row<B>(acc, ci, p, n, nn, zero, q, lane);
+    p += n;
     acc.fold();
     if (slot == 0) {
-      unsigned* p = s_part[l & 1][warp][sub];
-      p[0] = acc.a.lo; p[1] = acc.a.mid; p[2] = acc.a.hi;
-      p[3] = acc.b.lo; p[4] = acc.b.mid; p[5] = acc.b.hi;
+      unsigned* o = ends ? &s_sum[0][t * LPN + sub] : &s_piece[0][warp * LPN + sub];
+      const int st = ends ? kFxMaxRows<B> * LPN : kFxWarps * LPN;
+      o[0] = acc.a.lo; o[st] = acc.a.mid; o[2 * st] = acc.a.hi;
+      o[3 * st] = acc.b.lo; o[4 * st] = acc.b.mid; o[5 * st] = acc.b.hi;
     }
-    __syncthreads();
-    if (warp == l % kFxWarps && slot == 0) {
-      for (int w = 0; w < kFxWarps; ++w) {
-        if (w == warp) continue;
-        const unsigned* p = s_part[l & 1][w][sub];
-        acc.a.add(p[0], p[1], p[2]);
-        acc.b.add(p[3], p[4], p[5]);
+    if (!ends) {
+      tail = t;
+      break;
+    }
+    n = nn;
+    e = e2;
+  }
+  if (lane == 0) s_tail[warp] = tail;
+  __syncthreads();
+  // a thread per pair of columns of a row (an idle lane costs an FP64 slot too)
+  static_assert(kFxMaxRows<B> * LPN == kFxThreads, "one item a thread");
+  const int row = threadIdx.x / LPN;
+  if (row < nr) {
+    Acc<B> acc;
+    const int x = threadIdx.x;
+    acc.a = {s_sum[0][x], s_sum[1][x], s_sum[2][x]};
+    acc.b = {s_sum[3][x], s_sum[4][x], s_sum[5][x]};
+#pragma unroll
+    for (int w = 0; w < kFxWarps; ++w)
+      if (s_tail[w] == row) {
+        const int y2 = w * LPN + sub;
+        acc.a.add(s_piece[0][y2], s_piece[1][y2], s_piece[2][y2]);
+        acc.b.add(s_piece[3][y2], s_piece[4][y2], s_piece[5][y2]);
       }
-      const unsigned n = (unsigned)(e - s);
-      fx_store<B, SHIFT>(r0 + t, sub, acc.a.value(n, sa), acc.b.value(n, sb), out, scale, dshift, y);
-    }
+    const unsigned len = (unsigned)(s_off[row + 1] - s_off[row]);
+    fx_store<B, SHIFT>(r0 + row, sub, acc.a.value(len, fx_shift(ha)), acc.b.value(len, fx_shift(hb)), out, scale,
+                       dshift, y);
   }
 }
 
@@ -302,15 +328,24 @@ int launch_fx(int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_r
   SG_CHECK_LAUNCH();
   fx_quantize_kernel<B><<<grid_for(nvec, kFxThreads, 8 * sms), kFxThreads, 0, s>>>(nvec, v, head, q);
   SG_CHECK_LAUNCH();
-  int R = kFxWarps * (64 / B);
-  while (R > 4 && (rows + R - 1) / R < 8 * (int64_t)sms) R >>= 1;
+  // rows per CTA: the shortest schedule in waves of resident CTAs, a CTA's
+  // start counted as one row (5,000 equal rows as 1,250 CTAs on 608 places
+  // left the third wave nearly empty)
+  const int64_t slots = (int64_t)kFxCtas * sms;
+  int R = 1;
+  int64_t best = INT64_MAX;
+  for (int r = 1; r <= kFxMaxRows<B> && (r == 1 || r * in_rows <= INT32_MAX); ++r) {
+    const int64_t cost = ((rows + r - 1) / r + slots - 1) / slots * (r + 1);
+    if (cost < best) { best = cost; R = r; }
+  }
   const int64_t grid = (rows + R - 1) / R;
   if (grid > 0x7fffffffLL) return SG_ERR_ARG;
   if (dshift)
-    spmm_fx_kernel<B, true><<<(unsigned)grid, kFxThreads, 0, s>>>(rows, R, ptr, idx, in, q, head, out, scale, dshift, y);
+    spmm_fx_kernel<B, true><<<(unsigned)grid, kFxThreads, 0, s>>>(rows, R, (int)in_rows, ptr, idx, in, q, head, out, scale,
+                                                                  dshift, y);
   else
-    spmm_fx_kernel<B, false><<<(unsigned)grid, kFxThreads, 0, s>>>(rows, R, ptr, idx, in, q, head, out, scale, dshift,
-                                                                   y);
+    spmm_fx_kernel<B, false><<<(unsigned)grid, kFxThreads, 0, s>>>(rows, R, (int)in_rows, ptr, idx, in, q, head, out, scale,
+                                                                   dshift, y);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -322,14 +357,14 @@ using namespace sg;
 
 extern "C" int64_t sg_spmm_fx_work_bytes(int block, int64_t in_rows) {
   if (in_rows < 0 || (block != 4 && block != 8 && block != 16 && block != 32)) return -1;
-  return kHeadBytes + 8 * (int64_t)block * in_rows;
+  return kHeadBytes + 8 * (int64_t)block * (in_rows + 1);
 }
 
 extern "C" int sg_spmm_fx(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_rows,
                           const double* in, double* out, const double* scale, const double* dshift, const double* y,
                           void* work, int64_t work_bytes, void* stream) {
   const int64_t need = sg_spmm_fx_work_bytes(block, in_rows);
-  if (rows < 0 || need < 0 || !scale || (dshift && !y)) return SG_ERR_ARG;
+  if (rows < 0 || need < 0 || in_rows > INT32_MAX || !scale || (dshift && !y)) return SG_ERR_ARG;
   if (rows == 0) return SG_OK;
   if (!work || work_bytes < need) return SG_ERR_CAP;
   if (((uintptr_t)work | (uintptr_t)in | (uintptr_t)out | (uintptr_t)y) & 15u) return SG_ERR_ARG;

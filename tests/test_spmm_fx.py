@@ -100,3 +100,19 @@ def test_gpu_fixed_point_non_finite(bad):
     assert np.array_equal(np.isnan(got), np.isnan(plain)) and np.array_equal(np.isinf(got), np.isinf(plain))
     ok = np.isfinite(plain)
     assert np.allclose(got[ok], plain[ok], rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.parametrize("block", [4, 8, 16, 32])
+@pytest.mark.parametrize("rows,lengths", [(2, [20000, 1]), (9, [0, 0, 4097, 0, 31, 9000]), (64, [0]), (65, [1]),
+                                          (3001, [700, 0, 3, 2600, 33]), (5000, [0, 0, 0, 0, 0, 0, 0, 2000])])
+def test_gpu_fixed_point_rows_across_slices(block, rows, lengths):
+    """Rows that lie in several warps' slices, empty ones at the edges of a
+    slice and of a CTA: every row against the FP64 additions (their error is
+    at most len·2^-53 of Σ|terms|)."""
+    ptr, idx = _matrix(rows, 2000, rows, lengths)
+    X = np.random.default_rng(rows).standard_normal((2000, block))
+    scale = np.linspace(0.5, 2.0, rows)
+    got, plain = _run(block, ptr, idx, X, scale), _run(block, ptr, idx, X, scale, kernel="plain")
+    ln = np.diff(ptr)[:, None].astype(float)
+    tol = scale[:, None] * np.abs(X).max(axis=0)[None, :] * (ln * (ln + 4) * 2.0 ** -52 + ln * 2.0 ** -61)
+    assert np.all(np.abs(got - plain) <= tol)
