@@ -74,22 +74,29 @@ __global__ void select_fill(int64_t n, const int64_t* __restrict__ ptr, const in
 //   fill   : kTrRows rows at a time, in any order within them: every entry
 //            sets its row's bit in its column's mask, and after a barrier its
 //            place is the column's cursor plus the number of lower bits set;
-//            then the cursors move and the masks are cleared.  Rows ascend in every column whatever order the threads run
-//            in, so the result is identical run to run.
-// What bounds it: about 17 entries per (row, panel) at 500,000 columns, so the
+//            then the cursors move and the masks are cleared.  Rows ascend in
+//            every column whatever order the threads run in, so the result is
+//            identical run to run.
+// What bounds it: about 34 entries per (row, panel) at 500,000 columns, so the
 // work is short segments of dependent loads and shared-memory atomics.  The
 // form before took the rows of a block one at a time with a barrier after
 // each (136 of 512 threads busy: 9.9 ms of fill, 4.3 of count) and 304 row
 // blocks (2.6 ms for the offsets).  Half a warp per row segment, three barriers
-// per 128 rows and some 20 row blocks take 5.0 ms (fill), 1.2 (count) and 1.1
-// (segments, before 2.1) at 100,000 x 500,000 and 4.1e8 nonzeros; the fill is
-// bound by its scattered 4-byte stores (L1 and L2 at two thirds).  2,048 columns per panel keep the partly written sectors of
-// all resident CTAs (four per SM) at 40 MB of the 129 MB of L2.
+// per 128 rows and some 20 row blocks took 5.0 ms (fill), 1.2 (count) and 1.1
+// (segments, before 2.1) at 100,000 x 500,000 and 4.1e8 nonzeros with 2,048
+// columns per panel and 512 threads; 4,096 columns and 1,024 threads take 4.6,
+// 0.88 and 0.98 (8,192 columns and one CTA per SM 5.0, 0.88, 0.83; 256 rows per
+// step 5.1 and more; a whole warp per segment 5.0 and more).  The fill is
+// bound by its scattered 4-byte stores (L1 and L2 at two thirds); gathering a
+// column's rows in shared memory until a 32-byte sector is full took 12.5 ms
+// (the columns' unequal counts leave most lanes of a warp idle).  The partly
+// written sectors of all resident CTAs (two per SM) are 40 MB of the 129 MB of
+// L2.
 // ---------------------------------------------------------------------------
-constexpr int kTrLog = 11;
+constexpr int kTrLog = 12;
 constexpr int kTrPanel = 1 << kTrLog;
 constexpr int kTrRows = 128;             // rows per step of the fill: four mask words per column
-constexpr int kTrThreads = 512;
+constexpr int kTrThreads = 1024;
 constexpr int kTrHalf = 16;              // lanes per row segment
 constexpr int kTrSlots = kTrThreads / kTrHalf;  // segments at a time
 
@@ -196,7 +203,7 @@ __global__ void tr_offsets(int64_t m, int nblk, int32_t* __restrict__ cnt) {
   }
 }
 
-__global__ void __launch_bounds__(kTrThreads, 3)
+__global__ void __launch_bounds__(kTrThreads, 2)
 tr_fill(int64_t n, int64_t m, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
         const float* __restrict__ val, const int32_t* __restrict__ seg, int p0, int nblk,
         const int32_t* __restrict__ cnt, const int64_t* __restrict__ colptr, int32_t* __restrict__ rowidx, float* __restrict__ cval,
@@ -601,7 +608,7 @@ extern "C" int sg_csr_select_cols(int64_t n, const int64_t* indptr, const int32_
 
 extern "C" int sg_transpose_blocks(void) { return 2 * sm_count(); }
 
-// Row blocks of a transpose: eight waves of the four CTAs that an SM holds,
+// Row blocks of a transpose: sixteen waves of the two CTAs that an SM holds,
 // and at least one step of the fill per block.
 extern "C" int sg_transpose_row_blocks(int64_t n, int64_t m) {
   const int64_t P = (m + kTrPanel - 1) / kTrPanel;

@@ -1,5 +1,5 @@
 """The CSR -> CSC transpose (csrc/spectral.cu) against SciPy at the edges of
-its steps: panels of 2,048 columns, 128 rows per step and four 32-row mask
+its steps: panels of 4,096 columns, 128 rows per step and four 32-row mask
 words, row segments longer than the 16 lanes that share one, more row blocks
 than rows."""
 import numpy as np
@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,m,density,blocks", [(1, 1, 1.0, 1), (31, 2048, 1.0, 1), (127, 2047, 0.5, 3),
                                                 (128, 2049, 0.9, 1), (129, 4097, 0.05, 200), (700, 6000, 0.3, 2),
-                                                (5000, 300, 0.2, 7), (260, 70000, 0.01, 0)])
+                                                (5000, 300, 0.2, 7), (260, 70000, 0.01, 0), (300, 4095, 0.1, 2),
+                                                (257, 4096, 0.1, 1), (129, 8193, 0.2, 0)])
 @pytest.mark.parametrize("valued", [False, True])
 def test_gpu_transpose_edges(n, m, density, blocks, valued):
     import torch
