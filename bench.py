@@ -1230,7 +1230,7 @@ def run_import(args):
             "config": {"workload": f"{args.import_cells} cells, {lines} lines, {nbytes / 1e9:.2f} GB text, "
                                    "genome order, sorted_by_barcode=False, min_num_fragments=200",
                        "l2": "inputs larger than L2"},
-            "roofline": {"kernel": "whole import pipeline (parse, 3 radix sorts, segmented reductions)",
+            "roofline": {"kernel": "whole import pipeline (parse, hash grouping, radix sort by cell and chromosome)",
                          "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_kind, "traffic": None,
                          "algorithmic_bytes": alg, "note": "text read once + matrix and QC written once"},

@@ -388,7 +388,7 @@ __device__ __forceinline__ double hash_unit(uint64_t a, uint64_t b) {
 // into (ranks, lam), ascending (identity when sel is null).  One warp per
 // cluster of selected eigenvalues with consecutive ranks closer than
 // 1e-9 ‖T‖ (near-degenerate pairs).  Outside a cluster a converged vector is
-// within eps ‖T‖ / gap <= 2.2e-7 of its eigenvector, and orth_kernel then
+// within eps ‖T‖ / gap <= 2.2e-7 of its eigenvector, and orth_step_kernel then
 // restores orthonormality; LAPACK dstein clusters at 1e-3 ‖T‖ instead,
 // which chains the dense bulk of a Ritz spectrum (tiny eigenvalues 1e-7
 // apart) into long sequential runs.  Inside a cluster the vectors are done in

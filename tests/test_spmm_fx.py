@@ -1,7 +1,7 @@
 """FP64 SpMM by exact fixed-point sums (``sg_spmm_fx``) against correctly
-rounded row sums (``math.fsum``), at the edges of its row classes: empty
-rows, single chunks, the 512-nonzero bound above which a CTA shares a row,
-matrices short enough for the smallest CTA and long enough for the largest.
+rounded row sums (``math.fsum``): empty rows, single chunks, rows within one
+warp's slice and across several, matrices short enough for the smallest CTA
+and long enough for the largest.
 
 Bound, from the operand rounding (2^-62 of the column's largest magnitude a
 term, at most) and the few FP64 roundings of the epilogue:
