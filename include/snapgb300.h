@@ -383,6 +383,14 @@ int64_t sg_spmm_fx_work_bytes(int block, int64_t in_rows);
 int sg_spmm_fx(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_rows, const double* in,
                double* out, const double* scale, const double* dshift, const double* y, void* work,
                int64_t work_bytes, void* stream);
+/* The same for a matrix of counts: val holds whole numbers from 0 to 65,535 */
+/* with a row's sum below 2^32 (the caller checks: sg_counts_max writes the  */
+/* largest value, or 2^32 - 1 if one is not such a number).  No reference    */
+/* counterpart, as above.                                                    */
+int sg_spmm_fx_counts(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, const float* val,
+                      int64_t in_rows, const double* in, double* out, const double* scale, const double* dshift,
+                      const double* y, void* work, int64_t work_bytes, void* stream);
+int sg_counts_max(int64_t nnz, const float* val, uint32_t* out, void* stream);
 
 /* IDF weights from per-column cell counts (FP64, e.g. sg_col_counts of the */
 /* index pattern) with the rules of idf (embedding.rs:269-286): all counts   */

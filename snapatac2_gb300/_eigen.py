@@ -68,6 +68,7 @@ class GramOperator:
     staged_tables: dict = field(default_factory=dict)  # (pass, row bytes) -> segment table (uint8)
     counter: torch.Tensor | None = None  # row counters of the dynamically scheduled SpMM (one per pass)
     order_t: torch.Tensor | None = None  # int32 positions -> CSC rows, longest first (sg_row_order)
+    counts: bool | None = None  # holds_counts, once found
 
     def row_order_t(self, stream: int) -> torch.Tensor:
         """The CSC's rows (features) by descending length, dealt one per
@@ -83,6 +84,19 @@ class GramOperator:
                                       stream), "sg_row_order")
             self.order_t = order[:npos]
         return self.order_t
+
+    def holds_counts(self, stream: int) -> bool:
+        """Whether X's values are counts that the fixed-point sums can
+        multiply by: whole numbers from 0 to 65,535, and no row or column of
+        them can sum to 2^32.  Found once per operator."""
+        if self.counts is None:
+            top = torch.empty(1, dtype=torch.int64, device=self.a.device).zero_()
+            torch.cuda.current_stream(self.a.device).synchronize()
+            _lib.check(_lib.load().sg_counts_max(self.csr.data.numel(), self.csr.data.data_ptr(), top.data_ptr(),
+                                                 stream), "sg_counts_max")
+            torch.cuda.ExternalStream(stream, device=self.a.device).synchronize()
+            self.counts = int(top.item()) <= 65535 and int(top.item()) * max(self.n, self.m) < 1 << 32
+        return self.counts
 
     def scales(self, dtype_code: int):
         if dtype_code == 0:
@@ -116,8 +130,8 @@ class GramOperator:
             scale, dsh, yp = a.data_ptr(), dinv.data_ptr(), y.data_ptr()
             mask = self.row_mask.data_ptr() if self.row_mask is not None else None
         if variant >= FX:
-            if dtype_code == 1 and val is None and mask is None:
-                spmm_fx(rows, ptr, idx, cols, inp, out, scale, block, stream, dsh, yp)
+            if dtype_code == 1 and mask is None and (val is None or variant == FX_COUNTS and self.holds_counts(stream)):
+                spmm_fx(rows, ptr, idx, cols, inp, out, scale, block, stream, dsh, yp, val)
                 return _lib.SG_OK
             variant = 1
         if variant >= DYN and dtype_code != 0:
@@ -184,21 +198,30 @@ FP32_FLOOR = 3e-5
 
 # Variant codes >= STAGED select the stage-tiled SpMM kernel, codes >= DYN the
 # gather kernel on a persistent grid with dynamic row chunks (FP32), FX the
-# FP64 kernel with fixed-point sums (implicit ones, no mask).
+# FP64 kernel with fixed-point sums (implicit ones, no mask), FX_COUNTS the
+# same for values that are counts (GramOperator.holds_counts).
 STAGED = 100
 DYN = 200
 FX = 300
+FX_COUNTS = 301
 
 
 def spmm_fx(rows: int, ptr, idx, in_rows: int, inp, out, scale: int, block: int, stream: int, dshift=None,
-            y=None) -> None:
+            y=None, counts: int | None = None) -> None:
     """One FP64 SpMM of an implicit-ones CSR by exact fixed-point sums
-    (``sg_spmm_fx``); ``scale``, ``dshift`` and ``y`` are device addresses."""
+    (``sg_spmm_fx``), or of one whose values at ``counts`` are counts
+    (``sg_spmm_fx_counts``); ``scale``, ``dshift``, ``y`` and ``counts`` are
+    device addresses."""
     L = _lib.load()
     nb = int(L.sg_spmm_fx_work_bytes(block, in_rows))
     work = torch.empty(max(nb, 16), dtype=torch.uint8, device=inp.device)
     if stream != torch.cuda.current_stream(inp.device).cuda_stream:  # freed on the current stream, used on another
         work.record_stream(torch.cuda.ExternalStream(stream, device=inp.device))
+    if counts is not None:
+        _lib.check(L.sg_spmm_fx_counts(block, rows, ptr.data_ptr(), idx.data_ptr(), counts, in_rows, inp.data_ptr(),
+                                       out.data_ptr(), scale, dshift, y, work.data_ptr(), nb, stream),
+                   "sg_spmm_fx_counts")
+        return
     _lib.check(L.sg_spmm_fx(block, rows, ptr.data_ptr(), idx.data_ptr(), in_rows, inp.data_ptr(), out.data_ptr(),
                             scale, dshift, y, work.data_ptr(), nb, stream), "sg_spmm_fx")
 
@@ -229,19 +252,25 @@ def tune_spmm(op: "GramOperator", code: int, block: int, Z, Zs, T, W, stream: in
     SNAPGB300_SPMM_VARIANT=<t>,<x> (codes >= 100 select the staged kernel,
     >= 200 the dynamically scheduled gather kernel, 300 the fixed-point one).
 
-    FP64 without values or masks is not timed: the fixed-point kernel is the
-    faster one at every size measured (Xᵀ pass of 3.1e6 nonzeros, block 8:
-    39 us against 95; of 8.3e7, block 4: 0.39 ms against 0.97).
+    FP64 without values or masks, and with counts for values, is not timed:
+    the fixed-point kernel is the faster one at every size measured (Xᵀ pass
+    of 3.1e6 nonzeros, block 8: 38 us against 95; of 8.3e7, block 4: 0.34 ms
+    against 0.97; counts, 2.1e7 nonzeros, block 8: 191 us against 663).
     """
     import os
     forced = os.environ.get("SNAPGB300_SPMM_VARIANT")
     if forced:
         vt, vx = (int(x) for x in forced.split(","))
+        if op.csr.data is not None and FX_COUNTS in (vt, vx) and not op.holds_counts(stream):
+            vt, vx = (FX if v == FX_COUNTS else v for v in (vt, vx))  # the solver takes FP64 additions then
         op.variants[(code, block)] = (vt, vx)
         return vt, vx
     if code == 1 and op.csr.data is None and op.row_mask is None:
         op.variants[(code, block)] = (FX, FX)
         return FX, FX
+    if code == 1 and op.row_mask is None and op.holds_counts(stream):
+        op.variants[(code, block)] = (FX_COUNTS, FX_COUNTS)
+        return FX_COUNTS, FX_COUNTS
     key = (code, block, op.n, op.m, op.csr.nnz >> 20, op.csr.data is not None, op.row_mask is not None, staged)
     if key in _TUNED:
         op.variants[(code, block)] = _TUNED[key]
@@ -620,6 +649,8 @@ def _quick_variants(op: GramOperator, code: int, b: int, Z, Zs, T, W, stream: in
     else:
         if op.csr.data is None and op.row_mask is None:
             return FX, FX
+        if op.row_mask is None and op.holds_counts(stream):
+            return FX_COUNTS, FX_COUNTS
         cands = ([0, 1, 4, 5], [0, 1, 4, 5])
     best = []
     for which, cs in enumerate(cands):

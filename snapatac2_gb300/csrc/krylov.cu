@@ -29,6 +29,7 @@ namespace {
 constexpr int kStaged = 100;
 constexpr int kDyn = 200;
 constexpr int kFx = 300;  // FP64 fixed-point sums (implicit ones)
+constexpr int kFxCounts = 301;  // the same for values that the caller has found to be counts
 constexpr double kFp32Floor = 3e-5;  // residual level (x |A|) of a stalled FP32 solve
 
 // ---------------------------------------------------------------------------
@@ -349,6 +350,12 @@ struct Apply {
         ++spmm_launches;
         return sg_spmm_fx(B, rows, ptr, idx, t ? op->n : op->m, (const double*)in, (double*)out, (const double*)scale,
                           (const double*)dsh, (const double*)yy, fx, fx_bytes, s);
+      }
+      if (code && val && fx && variant == kFxCounts) {
+        launches += 3;
+        ++spmm_launches;
+        return sg_spmm_fx_counts(B, rows, ptr, idx, val, t ? op->n : op->m, (const double*)in, (double*)out,
+                                 (const double*)scale, (const double*)dsh, (const double*)yy, fx, fx_bytes, s);
       }
       variant = 1;
     }

@@ -1,5 +1,6 @@
-// FP64 SpMM of an implicit-ones CSR by exact fixed-point sums:
-//   out[r,:] = scale[r] * sum_{e in row r} in[col_e,:]  (- dshift[r] * y[r,:])
+// FP64 SpMM of an implicit-ones CSR, or of one that holds counts, by exact
+// fixed-point sums:
+//   out[r,:] = scale[r] * sum_{e in row r} val_e in[col_e,:]  (- dshift[r] * y[r,:])
 // for a dense block of B FP64 columns: the Gram matvec of the double-precision
 // solve (snapatac2-python/src/embedding.rs:133-152), the adjoint's passes and
 // the Nyström extension.
@@ -38,6 +39,14 @@
 // 5.9), where the 256-byte rows arrive at 22 / 19 TB/s.  (A warp per short row
 // and a CTA per long one: 167 / 159, 39 / 40, 390 / 430, 1,390 / 1,850.)  The
 // L1's lookups bind now (85-89 % of its peak throughput).
+//
+// Counts (COUNTS): a tile matrix holds whole numbers; an operand's integer
+// times a count below 2^16 is two wide integer multiplications, and with a
+// row's counts summing to less than 2^32 the 96 bits still hold every sum
+// exactly (the bias is taken out with the sum of the counts in place of the
+// row's length).  Three CTAs per SM (80 registers).  The same matrices with
+// counts 1 to 4: 191 / 152, 46 / 40 us, 0.38 / 0.35 and 1.61 / 1.68 ms (FP64
+// multiply-adds: 664 / 682, 121 / 118, 1.27 / 1.02, 8.36 / 8.04).
 #include "common.cuh"
 #include "internal.h"
 
@@ -47,6 +56,7 @@ namespace {
 constexpr int kFxThreads = 256;
 constexpr int kFxWarps = kFxThreads / 32;
 constexpr int kFxCtas = 4;       // CTAs per SM (64 registers)
+constexpr int kFxCtasCounts = 3;
 template <int B>
 constexpr int kFxMaxRows = kFxWarps * (64 / B);  // rows per CTA at most
 constexpr int kHeadBytes = 256;    // per-column maxima in front of the integers
@@ -107,6 +117,18 @@ fx_quantize_kernel(int64_t nvec, const double2* __restrict__ in, const unsigned*
   }
 }
 
+// the largest of val, all of them whole numbers from 0 to 65,535, else 2^32 - 1
+__global__ void __launch_bounds__(kFxThreads)
+counts_max_kernel(int64_t nnz, const float* __restrict__ val, uint32_t* __restrict__ out) {
+  unsigned m = 0;
+  for (int64_t i = blockIdx.x * (int64_t)kFxThreads + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * kFxThreads) {
+    const float v = val[i];
+    m = max(m, v >= 0.f && v <= 65535.f && v == truncf(v) ? (unsigned)v : 0xffffffffu);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
 struct Sum96 {
   unsigned lo, mid, hi;
   __device__ __forceinline__ void add(unsigned l, unsigned m) {
@@ -128,10 +150,23 @@ struct Sum96 {
   }
 };
 
-template <int B>
+// v times the 64-bit integer (v below 2^16)
+__device__ __forceinline__ void add_times(Sum96& s, unsigned long long g, unsigned v) {
+  const unsigned long long p = (unsigned long long)(unsigned)g * v;
+  const unsigned long long r = (g >> 32) * v + (p >> 32);
+  s.add((unsigned)p, (unsigned)r, (unsigned)(r >> 32));
+}
+
+template <int B, bool COUNTS>
 struct Acc {
   Sum96 a, b;  // the lane's two columns
-  __device__ __forceinline__ void zero() { a = {0, 0, 0}; b = {0, 0, 0}; }
+  unsigned n;  // COUNTS: the sum of the counts
+  __device__ __forceinline__ void zero() { a = {0, 0, 0}; b = {0, 0, 0}; n = 0; }
+  __device__ __forceinline__ void add(const ulonglong2& g, unsigned v) {
+    add_times(a, g.x, v);
+    add_times(b, g.y, v);
+    n += v;
+  }
   __device__ __forceinline__ void add(const ulonglong2& g) {
     a.add((unsigned)g.x, (unsigned)(g.x >> 32));
     b.add((unsigned)g.y, (unsigned)(g.y >> 32));
@@ -145,6 +180,7 @@ struct Acc {
                      y2 = __shfl_xor_sync(0xffffffffu, b.hi, o);
       a.add(x0, x1, x2);
       b.add(y0, y1, y2);
+      if (COUNTS) n += __shfl_xor_sync(0xffffffffu, n, o);
     }
   }
 };
@@ -157,9 +193,17 @@ __device__ __forceinline__ void fx_load(int (&ci)[CH], const int32_t* __restrict
   for (int c = 0; c < CH; ++c) ci[c] = c * 32 + lane < n ? __ldg(p + c * 32 + lane) : zero;
 }
 
-// adds the rows named by the first N chunks of ci
-template <int B, int CH, int N>
-__device__ __forceinline__ void fx_add(Acc<B>& acc, const int (&ci)[CH], const ulonglong2* __restrict__ q, int lane) {
+// their counts (0 past them)
+template <int CH>
+__device__ __forceinline__ void fx_load_counts(float (&cv)[CH], const float* __restrict__ p, int n, int lane) {
+#pragma unroll
+  for (int c = 0; c < CH; ++c) cv[c] = c * 32 + lane < n ? __ldg(p + c * 32 + lane) : 0.f;
+}
+
+// adds the rows named by the first N chunks of ci (COUNTS: cv times each)
+template <int B, int CH, int N, bool COUNTS>
+__device__ __forceinline__ void fx_add(Acc<B, COUNTS>& acc, const int (&ci)[CH], const float (&cv)[CH],
+                                       const ulonglong2* __restrict__ q, int lane) {
   constexpr int LPN = B / 2, NPS = 32 / LPN;
   constexpr int GB = LPN < 8 ? LPN : 8;  // gathers in flight per chunk
   const int sub = lane % LPN, slot = lane / LPN;
@@ -174,7 +218,12 @@ __device__ __forceinline__ void fx_add(Acc<B>& acc, const int (&ci)[CH], const u
         g[c * GB + j] = __ldg(q + (uint64_t)col * LPN + sub);
       }
 #pragma unroll
-    for (int t = 0; t < N * GB; ++t) acc.add(g[t]);
+    for (int t = 0; t < N * GB; ++t) {
+      if constexpr (COUNTS)
+        acc.add(g[t], __shfl_sync(0xffffffffu, (unsigned)cv[t / GB], (j0 + t % GB) * NPS + slot));
+      else
+        acc.add(g[t]);
+    }
   }
 }
 
@@ -185,20 +234,29 @@ constexpr int kChunks = B == 4 ? 4 : (B == 8 ? 2 : 1);
 // chunks and receives those of the next nn nonzeros after the row (the warp's
 // next row).  Indices are loaded one step ahead, so a step waits for the
 // gathers alone.
-template <int B>
-__device__ __forceinline__ void fx_row(Acc<B>& acc, int (&ci)[kChunks<B>], const int32_t* __restrict__ p, int n,
-                                       int nn, int zero, const ulonglong2* __restrict__ q, int lane) {
+template <int B, bool COUNTS>
+__device__ __forceinline__ void fx_row(Acc<B, COUNTS>& acc, int (&ci)[kChunks<B>], float (&cv)[kChunks<B>],
+                                       const int32_t* __restrict__ p, const float* __restrict__ pv, int n, int nn,
+                                       int zero, const ulonglong2* __restrict__ q, int lane) {
   constexpr int CH = kChunks<B>, STEP = 32 * CH;
   while (n > 0) {
     int next[CH];
+    float nextv[CH];
     const int adv = n < STEP ? n : STEP;
     p += adv;
     fx_load<CH>(next, p, n > STEP ? n - STEP : nn, zero, lane);
-    if (CH == 1 || n > 16 * CH) fx_add<B, CH, CH>(acc, ci, q, lane);
-    else if (CH == 4 && n > 32) fx_add<B, CH, CH == 4 ? 2 : 1>(acc, ci, q, lane);
-    else fx_add<B, CH, 1>(acc, ci, q, lane);
+    if (COUNTS) {
+      pv += adv;
+      fx_load_counts<CH>(nextv, pv, n > STEP ? n - STEP : nn, lane);
+    }
+    if (CH == 1 || n > 16 * CH) fx_add<B, CH, CH>(acc, ci, cv, q, lane);
+    else if (CH == 4 && n > 32) fx_add<B, CH, CH == 4 ? 2 : 1>(acc, ci, cv, q, lane);
+    else fx_add<B, CH, 1>(acc, ci, cv, q, lane);
 #pragma unroll
-    for (int c = 0; c < CH; ++c) ci[c] = next[c];
+    for (int c = 0; c < CH; ++c) {
+      ci[c] = next[c];
+      if (COUNTS) cv[c] = nextv[c];
+    }
     n -= STEP;
   }
 }
@@ -221,17 +279,19 @@ __device__ __forceinline__ void fx_store(int64_t r, int sub, double a, double b,
   *reinterpret_cast<double2*>(out + r * B + 2 * sub) = o;
 }
 
-template <int B, bool SHIFT>
-__global__ void __launch_bounds__(kFxThreads, kFxCtas)
+template <int B, bool SHIFT, bool COUNTS>
+__global__ void __launch_bounds__(kFxThreads, COUNTS ? kFxCtasCounts : kFxCtas)
 spmm_fx_kernel(int64_t rows, int R, int zero, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+               const float* __restrict__ val,
                const double* __restrict__ in, const ulonglong2* __restrict__ q, const unsigned* __restrict__ head,
                double* __restrict__ out, const double* __restrict__ scale, const double* __restrict__ dshift,
                const double* __restrict__ y) {
   constexpr int LPN = B / 2, NPS = 32 / LPN;
   constexpr int CH = kChunks<B>;
   __shared__ int s_off[kFxMaxRows<B> + 2];  // row offsets in the CTA's nonzeros (below 2^31), the last one twice
-  __shared__ unsigned s_sum[6][kFxMaxRows<B> * LPN];  // of the rows, less the pieces in s_piece
-  __shared__ unsigned s_piece[6][kFxWarps * LPN];     // a warp's piece of the row that its slice ends inside of
+  constexpr int NW = COUNTS ? 7 : 6;
+  __shared__ unsigned s_sum[NW][kFxMaxRows<B> * LPN];  // of the rows, less the pieces in s_piece
+  __shared__ unsigned s_piece[NW][kFxWarps * LPN];    // a warp's piece of the row that its slice ends inside of
   __shared__ int s_tail[kFxWarps];                    // that row, or -1
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane % LPN, slot = lane / LPN;
@@ -240,6 +300,7 @@ spmm_fx_kernel(int64_t rows, int R, int zero, const int64_t* __restrict__ ptr, c
   const int64_t p0 = ptr[r0];
   if (threadIdx.x <= nr + 1) s_off[threadIdx.x] = (int)(ptr[r0 + min((int)threadIdx.x, nr)] - p0);
   idx += p0;
+  if (COUNTS) val += p0;
   const unsigned ha = head[2 * sub], hb = head[2 * sub + 1];
   const bool finite = __all_sync(0xffffffffu, ha < kNonFinite && hb < kNonFinite);  // the same in every warp
   __syncthreads();
@@ -247,7 +308,8 @@ spmm_fx_kernel(int64_t rows, int R, int zero, const int64_t* __restrict__ ptr, c
     for (int i = warp; i < nr; i += kFxWarps) {
       double2 acc = make_double2(0.0, 0.0);
       for (int k = s_off[i] + slot; k < s_off[i + 1]; k += NPS)
-        V16<double>::add(acc, *reinterpret_cast<const double2*>(in + (int64_t)idx[k] * B + 2 * sub));
+        V16<double>::fma(acc, COUNTS ? (double)val[k] : 1.0,
+                         *reinterpret_cast<const double2*>(in + (int64_t)idx[k] * B + 2 * sub));
       __syncwarp();
 #pragma unroll
       for (int o = LPN; o < 32; o <<= 1) V16<double>::add(acc, V16<double>::shfl_xor(acc, o));
@@ -265,22 +327,31 @@ spmm_fx_kernel(int64_t rows, int R, int zero, const int64_t* __restrict__ ptr, c
   const int32_t* p = idx + sl;
   int ci[CH], e = s_off[min(t, nr) + 1], n = t < nr ? min(e, sh) - sl : 0;
   int tail = -1;
+  const float* pv = COUNTS ? val + sl : nullptr;
+  float cv[CH];
   fx_load<CH>(ci, p, n, zero, lane);
+  if (COUNTS) fx_load_counts<CH>(cv, pv, n, lane);
   for (; t < nr; ++t) {
     const bool ends = e <= sh;
     if (!ends && n == 0) break;
     const int e2 = s_off[t + 2], nn = min(e2, sh) - min(e, sh);
-    Acc<B> acc;
+    Acc<B, COUNTS> acc;
     acc.zero();
-    if (n == 0) fx_load<CH>(ci, p, nn, zero, lane);
-    else fx_row<B>(acc, ci, p, n, nn, zero, q, lane);
+    if (n == 0) {
+      fx_load<CH>(ci, p, nn, zero, lane);
+      if (COUNTS) fx_load_counts<CH>(cv, pv, nn, lane);
+    } else {
+      fx_row<B, COUNTS>(acc, ci, cv, p, pv, n, nn, zero, q, lane);
+    }
     p += n;
+    if (COUNTS) pv += n;
     acc.fold();
     if (slot == 0) {
       unsigned* o = ends ? &s_sum[0][t * LPN + sub] : &s_piece[0][warp * LPN + sub];
       const int st = ends ? kFxMaxRows<B> * LPN : kFxWarps * LPN;
       o[0] = acc.a.lo; o[st] = acc.a.mid; o[2 * st] = acc.a.hi;
       o[3 * st] = acc.b.lo; o[4 * st] = acc.b.mid; o[5 * st] = acc.b.hi;
+      if (COUNTS) o[6 * st] = acc.n;
     }
     if (!ends) {
       tail = t;
@@ -295,25 +366,27 @@ spmm_fx_kernel(int64_t rows, int R, int zero, const int64_t* __restrict__ ptr, c
   static_assert(kFxMaxRows<B> * LPN == kFxThreads, "one item a thread");
   const int row = threadIdx.x / LPN;
   if (row < nr) {
-    Acc<B> acc;
+    Acc<B, COUNTS> acc;
     const int x = threadIdx.x;
     acc.a = {s_sum[0][x], s_sum[1][x], s_sum[2][x]};
     acc.b = {s_sum[3][x], s_sum[4][x], s_sum[5][x]};
+    acc.n = COUNTS ? s_sum[NW - 1][x] : 0;
 #pragma unroll
     for (int w = 0; w < kFxWarps; ++w)
       if (s_tail[w] == row) {
         const int y2 = w * LPN + sub;
         acc.a.add(s_piece[0][y2], s_piece[1][y2], s_piece[2][y2]);
         acc.b.add(s_piece[3][y2], s_piece[4][y2], s_piece[5][y2]);
+        if (COUNTS) acc.n += s_piece[NW - 1][y2];
       }
-    const unsigned len = (unsigned)(s_off[row + 1] - s_off[row]);
+    const unsigned len = COUNTS ? acc.n : (unsigned)(s_off[row + 1] - s_off[row]);
     fx_store<B, SHIFT>(r0 + row, sub, acc.a.value(len, fx_shift(ha)), acc.b.value(len, fx_shift(hb)), out, scale,
                        dshift, y);
   }
 }
 
 template <int B>
-int launch_fx(int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_rows, const double* in, double* out,
+int launch_fx(int64_t rows, const int64_t* ptr, const int32_t* idx, const float* val, int64_t in_rows, const double* in, double* out,
               const double* scale, const double* dshift, const double* y, char* work, cudaStream_t s) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -331,7 +404,7 @@ int launch_fx(int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_r
   // rows per CTA: the shortest schedule in waves of resident CTAs, a CTA's
   // start counted as one row (5,000 equal rows as 1,250 CTAs on 608 places
   // left the third wave nearly empty)
-  const int64_t slots = (int64_t)kFxCtas * sms;
+  const int64_t slots = (int64_t)(val ? kFxCtasCounts : kFxCtas) * sms;
   int R = 1;
   int64_t best = INT64_MAX;
   for (int r = 1; r <= kFxMaxRows<B> && (r == 1 || r * in_rows <= INT32_MAX); ++r) {
@@ -340,12 +413,16 @@ int launch_fx(int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_r
   }
   const int64_t grid = (rows + R - 1) / R;
   if (grid > 0x7fffffffLL) return SG_ERR_ARG;
-  if (dshift)
-    spmm_fx_kernel<B, true><<<(unsigned)grid, kFxThreads, 0, s>>>(rows, R, (int)in_rows, ptr, idx, in, q, head, out, scale,
-                                                                  dshift, y);
-  else
-    spmm_fx_kernel<B, false><<<(unsigned)grid, kFxThreads, 0, s>>>(rows, R, (int)in_rows, ptr, idx, in, q, head, out, scale,
-                                                                   dshift, y);
+  auto run = [&](auto kern) {
+    kern<<<(unsigned)grid, kFxThreads, 0, s>>>(rows, R, (int)in_rows, ptr, idx, val, in, q, head, out, scale, dshift, y);
+  };
+  if (val) {
+    if (dshift) run(spmm_fx_kernel<B, true, true>);
+    else run(spmm_fx_kernel<B, false, true>);
+  } else {
+    if (dshift) run(spmm_fx_kernel<B, true, false>);
+    else run(spmm_fx_kernel<B, false, false>);
+  }
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -360,9 +437,10 @@ extern "C" int64_t sg_spmm_fx_work_bytes(int block, int64_t in_rows) {
   return kHeadBytes + 8 * (int64_t)block * (in_rows + 1);
 }
 
-extern "C" int sg_spmm_fx(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_rows,
-                          const double* in, double* out, const double* scale, const double* dshift, const double* y,
-                          void* work, int64_t work_bytes, void* stream) {
+namespace {
+int spmm_fx_any(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, const float* val, int64_t in_rows,
+                const double* in, double* out, const double* scale, const double* dshift, const double* y, void* work,
+                int64_t work_bytes, void* stream) {
   const int64_t need = sg_spmm_fx_work_bytes(block, in_rows);
   if (rows < 0 || need < 0 || in_rows > INT32_MAX || !scale || (dshift && !y)) return SG_ERR_ARG;
   if (rows == 0) return SG_OK;
@@ -371,9 +449,34 @@ extern "C" int sg_spmm_fx(int block, int64_t rows, const int64_t* ptr, const int
   cudaStream_t s = as_stream(stream);
   char* w = reinterpret_cast<char*>(work);
   switch (block) {
-    case 4: return launch_fx<4>(rows, ptr, idx, in_rows, in, out, scale, dshift, y, w, s);
-    case 8: return launch_fx<8>(rows, ptr, idx, in_rows, in, out, scale, dshift, y, w, s);
-    case 16: return launch_fx<16>(rows, ptr, idx, in_rows, in, out, scale, dshift, y, w, s);
-    default: return launch_fx<32>(rows, ptr, idx, in_rows, in, out, scale, dshift, y, w, s);
+    case 4: return launch_fx<4>(rows, ptr, idx, val, in_rows, in, out, scale, dshift, y, w, s);
+    case 8: return launch_fx<8>(rows, ptr, idx, val, in_rows, in, out, scale, dshift, y, w, s);
+    case 16: return launch_fx<16>(rows, ptr, idx, val, in_rows, in, out, scale, dshift, y, w, s);
+    default: return launch_fx<32>(rows, ptr, idx, val, in_rows, in, out, scale, dshift, y, w, s);
   }
+}
+}  // namespace
+
+extern "C" int sg_spmm_fx(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, int64_t in_rows,
+                          const double* in, double* out, const double* scale, const double* dshift, const double* y,
+                          void* work, int64_t work_bytes, void* stream) {
+  return spmm_fx_any(block, rows, ptr, idx, nullptr, in_rows, in, out, scale, dshift, y, work, work_bytes, stream);
+}
+
+extern "C" int sg_spmm_fx_counts(int block, int64_t rows, const int64_t* ptr, const int32_t* idx, const float* val,
+                                 int64_t in_rows, const double* in, double* out, const double* scale,
+                                 const double* dshift, const double* y, void* work, int64_t work_bytes,
+                                 void* stream) {
+  if (!val) return SG_ERR_ARG;
+  return spmm_fx_any(block, rows, ptr, idx, val, in_rows, in, out, scale, dshift, y, work, work_bytes, stream);
+}
+
+extern "C" int sg_counts_max(int64_t nnz, const float* val, uint32_t* out, void* stream) {
+  if (nnz < 0 || !out || (nnz > 0 && !val)) return SG_ERR_ARG;
+  cudaStream_t s = as_stream(stream);
+  if (cudaMemsetAsync(out, 0, sizeof(uint32_t), s) != cudaSuccess) return SG_ERR_CUDA;
+  if (nnz == 0) return SG_OK;
+  counts_max_kernel<<<grid_for(nnz, kFxThreads * 8, 16384), kFxThreads, 0, s>>>(nnz, val, out);
+  SG_CHECK_LAUNCH();
+  return SG_OK;
 }

@@ -116,3 +116,76 @@ def test_gpu_fixed_point_rows_across_slices(block, rows, lengths):
     ln = np.diff(ptr)[:, None].astype(float)
     tol = scale[:, None] * np.abs(X).max(axis=0)[None, :] * (ln * (ln + 4) * 2.0 ** -52 + ln * 2.0 ** -61)
     assert np.all(np.abs(got - plain) <= tol)
+
+
+@pytest.mark.parametrize("block", [4, 8, 16, 32])
+@pytest.mark.parametrize("rows,lengths,top", [(3, [0, 1, 900], 1), (40, [5, 64, 65, 0, 700], 4),
+                                              (300, [2000, 1, 33], 65535), (5000, [0, 3, 40, 9], 7)])
+def test_gpu_fixed_point_counts(block, rows, lengths, top):
+    """Values that are counts (sg_spmm_fx_counts) against exact sums: bound as
+    above with Σ counts in place of the row's length."""
+    import torch
+    from snapatac2_gb300 import _lib
+    L = _lib.lib()
+    ptr, idx = _matrix(rows, 3000, rows, lengths)
+    rng = np.random.default_rng(rows + block)
+    X = rng.standard_normal((3000, block)) * np.exp(rng.standard_normal((3000, block)))
+    val = rng.integers(0, top + 1, idx.size).astype(np.float32)
+    val[-1] = top
+    scale, dsh, y = rng.random(rows) + 0.5, rng.random(rows), rng.standard_normal((rows, block))
+    t = [torch.from_numpy(a).cuda() for a in (ptr, idx, val, X, scale, dsh, y)]
+    out = torch.full((rows, block), 7.0, dtype=torch.float64, device="cuda")
+    nb = int(L.sg_spmm_fx_work_bytes(block, 3000))
+    work = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    sh = torch.cuda.current_stream().cuda_stream
+    q = [a.data_ptr() for a in t]
+    _lib.check(L.sg_spmm_fx_counts(block, rows, q[0], q[1], q[2], 3000, q[3], out.data_ptr(), q[4], q[5], q[6],
+                                   work.data_ptr(), nb, sh), "counts")
+    got, m = out.cpu().numpy(), np.abs(X).max(axis=0)
+    for r in list(range(min(rows, 60))) + [rows - 1]:
+        e, v = idx[ptr[r]:ptr[r + 1]], val[ptr[r]:ptr[r + 1]].astype(float)
+        for c in range(block):
+            # count x operand split at 26 bits is exact in parts
+            hi = np.float64(np.float32(X[e, c]))
+            s = math.fsum(np.concatenate([v * hi, v * (X[e, c] - hi)]))
+            bound = v.sum() * 2.0 ** -62 * m[c] * scale[r] + 2.0 ** -51 * (abs(scale[r] * s) + abs(dsh[r] * y[r, c]))
+            assert abs(got[r, c] - (scale[r] * s - dsh[r] * y[r, c])) <= bound + 1e-320, (r, c)
+    mx = torch.zeros(1, dtype=torch.int64, device="cuda")
+    for bad, want in ((None, top), (0.5, 2 ** 32 - 1), (-1.0, 2 ** 32 - 1), (65536.0, 2 ** 32 - 1),
+                      (np.nan, 2 ** 32 - 1)):
+        w = val.copy()
+        if bad is not None:
+            w[w.size // 2] = bad
+        d = torch.from_numpy(w).cuda()
+        _lib.check(L.sg_counts_max(w.size, d.data_ptr(), mx.data_ptr(), sh), "max")
+        assert int(mx) == want
+
+
+@pytest.mark.parametrize("fraction", [False, True])
+def test_gpu_counts_take_the_fixed_point_kernel(fraction):
+    """An FP64 solve of a matrix of counts against the FP64 additions, and one
+    with a fractional value, which keeps them."""
+    import torch
+    from snapatac2_gb300 import _eigen
+    import scipy.sparse as sp
+    from snapatac2_gb300._binning import DeviceCSR
+    rng = np.random.default_rng(3)
+    A = sp.random(400, 3000, density=0.05, format="csr", random_state=1)
+    A.sort_indices()
+    A.data = rng.integers(1, 5, A.nnz).astype(np.float32)
+    if fraction:
+        A.data[7] = 1.5
+    d = lambda a, t: torch.from_numpy(np.ascontiguousarray(a.astype(t))).cuda()  # noqa: E731
+    csr = DeviceCSR(d(A.indptr, np.int64), d(A.indices, np.int32), d(A.data, np.float32), A.shape)
+    op = _eigen.build_operator(csr)
+    sh = torch.cuda.current_stream().cuda_stream
+    assert op.holds_counts(sh) is (not fraction)
+    z = torch.from_numpy(rng.standard_normal((400, 8))).cuda()
+    zs, t, w = op.a[:, None] * z, torch.empty(3000, 8, dtype=torch.float64, device="cuda"), torch.empty_like(z)
+    ref_t, ref = torch.empty_like(t), torch.empty_like(w)
+    op.apply(1, 8, z, zs, t, w, sh)
+    assert op.variants[(1, 8)][0] == _eigen.FX_COUNTS if not fraction else op.variants[(1, 8)][0] < _eigen.FX
+    op.spmm_pass(0, 1, 1, 8, zs, ref_t, sh)
+    op.spmm_pass(1, 1, 1, 8, ref_t, ref, sh, z)
+    assert float((t - ref_t).abs().max() / ref_t.abs().max()) < 1e-13
+    assert float((w - ref).abs().max() / ref.abs().max()) < 1e-13
