@@ -374,8 +374,10 @@ int sg_spmm_masked(int dtype, int block, int64_t rows, const int64_t* ptr, const
 /* exact fixed-point sums: each column of `in` (in_rows x block) is scaled by */
 /* a power of two, rounded once to 64-bit integers (error <= 2^-62 of the    */
 /* column's largest magnitude) and summed in 96 bits, so the sums do not     */
-/* depend on their order.  A non-finite value in `in` sends the call through */
-/* FP64 additions.  work: sg_spmm_fx_work_bytes(block, in_rows) bytes of     */
+/* depend on their order.  Row sums for which that could be less accurate    */
+/* than FP64 additions (every operand below about 2^-8 of its column's       */
+/* largest) are taken by FP64 additions, as is every row when `in` holds a   */
+/* non-finite value.  work: sg_spmm_fx_work_bytes(block, in_rows) bytes of   */
 /* device scratch, one per concurrent call; in / out / y / work 16-byte      */
 /* aligned.  No reference counterpart (an arithmetic form of the FP64        */
 /* matvec of embedding.rs:155-188).                                          */
