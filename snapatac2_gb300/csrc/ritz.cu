@@ -46,6 +46,10 @@ namespace {
 
 constexpr int kTriThreads = 256;
 constexpr int kMaxCluster = 16;
+// The reduction forms products of three entries of the matrix (uᵀv), so it
+// runs on entries scaled by a power of two when the largest is not within
+// 2^±kTriRange (d and e are scaled back).
+constexpr int kTriRange = 100;
 
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
@@ -97,14 +101,35 @@ tridiag_kernel(int n, const double* __restrict__ A, int64_t lda, double* __restr
   double* ub = vb + 2 * n;
   double* slots = ub + 2 * n;
   double* red = slots + 2 * kMaxCluster * kTriWarps;
-  double* sc = red + kTriWarps;  // 0: K, 1: w_j, 2: μ (μ + |α|), 3: τ
+  double* sc = red + kTriWarps;  // 0: K, 1: w_j, 2: μ (μ + |α|), 3: τ, 4: the scaling back
   constexpr int kSlots = CS * kTriWarps, kPer = (kRitzMaxN + kTriThreads - 1) / kTriThreads;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned top = 0;  // high word of the largest |A_ij| of this CTA's rows
   for (int t = threadIdx.x; t < R * n; t += blockDim.x) {
     const int li = t / n, c = t % n;
     const int i = li * CS + rank;
-    Al[t] = i < n ? A[(int64_t)i * lda + c] : 0.0;
+    const double x = i < n ? A[(int64_t)i * lda + c] : 0.0;
+    Al[t] = x;
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    top = h > top ? h : top;
   }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) slots[warp] = __hiloint2double((int)top, 0);
+  if (CS > 1) cl.sync(); else __syncthreads();
+  top = 0;
+  for (int q = lane; q < kSlots; q += 32) {
+    const double* other = CS > 1 ? cl.map_shared_rank(slots, q / kTriWarps) : slots;
+    top = max(top, (unsigned)__double2hiint(other[q % kTriWarps]));
+  }
+  top = __reduce_max_sync(0xffffffffu, top);  // the same in every warp of the cluster
+  double back = 1.0;
+  if (top < (1023u - kTriRange) << 20 || (top >= (1023u + kTriRange) << 20 && top < 0x7ff00000u)) {
+    const int te = (int)(top >> 20), up = max(min(1023 - te, 1000), -1022);  // the largest entry to about 1
+    const double f = __longlong_as_double((long long)(1023 + up) << 52);
+    back = __longlong_as_double((long long)(1023 - up) << 52);
+    for (int t = threadIdx.x; t < R * n; t += blockDim.x) Al[t] *= f;
+  }
+  if (threadIdx.x == 0) sc[4] = back;
   if (CS > 1) cl.sync(); else __syncthreads();
   // steps 0 .. n-3 make reflectors; step n-2 only finishes the last 2 x 2 block
   for (int j = 0; j + 1 < n; ++j) {
@@ -163,17 +188,18 @@ tridiag_kernel(int n, const double* __restrict__ A, int64_t lda, double* __restr
       if (lane == 0) {
         const double alpha = v[j + 1];
         double beta = alpha, den = 0.0;
-        if (sigma > 0.0) {
+        const double x = fma(alpha, alpha, sigma);
+        if (sigma > 0.0 && x >= 0x1p-1000) {  // below, the row is done: 2^-400 of the matrix at most
           // x rsqrt(x): 350 + 64 clocks of this chain, a square root 675
-          const double x = fma(alpha, alpha, sigma), mu = x * rsqrt(x);
+          const double mu = x * rsqrt(x);
           beta = alpha <= 0.0 ? mu : -mu;
           den = mu * (mu + fabs(alpha));
           v[j + 1] = alpha - beta;
         }
         sc[2] = den;
         if (rank == j % CS) {
-          d[j] = v[j];
-          e[j] = beta;
+          d[j] = v[j] * sc[4];
+          e[j] = beta * sc[4];
         }
       }
     }
@@ -220,15 +246,15 @@ tridiag_kernel(int n, const double* __restrict__ A, int64_t lda, double* __restr
     double x = row[n - 1];
     if (n >= 2) {
       const double* v = vb + ((n - 2) & 1) * n;
-      d[n - 2] = v[n - 2];
-      e[n - 2] = v[n - 1];
+      d[n - 2] = v[n - 2] * sc[4];
+      e[n - 2] = v[n - 1] * sc[4];
       tau[n - 2] = 0.0;
       if (n >= 3) {
         const double vl = vb[((n - 3) & 1) * n + n - 1], wl = ub[((n - 3) & 1) * n + n - 1];
         x = fma(-vl, wl, fma(-wl, vl, x));
       }
     }
-    d[n - 1] = x;
+    d[n - 1] = x * sc[4];
     tau[n - 1] = 0.0;
   }
   if (CS > 1) cl.sync();
