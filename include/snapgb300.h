@@ -534,6 +534,14 @@ int64_t sg_sym_eig_work_bytes(int n, int p, int q);
 int sg_sym_eig(int n, const double* A, int64_t lda, int p, int q, double* evals, double* evecs, void* work,
                int64_t work_bytes, void* stream);
 
+/* Its last step: the nw rows of Z (length n, nw <= n <= 640) to an          */
+/* orthonormal set of the same span, the closest one where they are near     */
+/* orthonormal already, in place.  Rows of about unit length; work: 8-byte   */
+/* aligned.  Replaces the orthogonality that ARPACK's eigensolve returns     */
+/* (embedding.rs:155-171).                                                   */
+int64_t sg_orth_rows_work_bytes(int nw, int n);
+int sg_orth_rows(int nw, int n, double* Z, void* work, int64_t work_bytes, void* stream);
+
 /* ---- one-call eigensolver: replaces eigen (embedding.rs:155-188) ------- */
 /* The operator A v = a ⊙ (X (w² ⊙ (Xᵀ (a ⊙ v)))) - dinv ⊙ v of one dataset, */
 /* as sg_csr_transpose and sg_spectral_prepare leave it; the reference       */

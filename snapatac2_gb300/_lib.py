@@ -134,6 +134,8 @@ SIGNATURES: dict[str, tuple] = {
                                     _P, _P, _P]),
     "sg_sym_eig_work_bytes": (_I64, [_I32, _I32, _I32]),
     "sg_sym_eig": (_I32, [_I32, _P, _I64, _I32, _I32, _P, _P, _P, _I64, _P]),
+    "sg_orth_rows_work_bytes": (_I64, [_I32, _I32]),
+    "sg_orth_rows": (_I32, [_I32, _I32, _P, _P, _I64, _P]),
     "sg_lanczos_work_bytes": (_I64, [_I32, _I32, _I32, _I64, _I64, _I32, _I32]),
     "sg_lanczos": (_I32, [_P, _I32, _I32, _I32, ctypes.c_uint64, _P, _P, _I64, _P, _P, _P, _P, _P, _P]),
 }
@@ -176,7 +178,7 @@ KERNELS_PER_CALL = {
     "sg_square_values": 1,
     "sg_frag_count_lines": 4, "sg_frag_index_lines": 1, "sg_region_plan": 4, "sg_region_run": 5, "sg_region_index": 2, "sg_region_plan_indexed": 4, "sg_region_run_indexed": 5,
     "sg_csr_row_ptr": 4, "sg_csr_copy_rows": 1, "sg_gather_bytes": 1, "sg_nystrom_rescale": 1,
-    "sg_sym_eig": 11, "sg_csr_aggregate_count": 2, "sg_csr_aggregate_run": 14,
+    "sg_sym_eig": 11, "sg_orth_rows": 5, "sg_csr_aggregate_count": 2, "sg_csr_aggregate_run": 14,
 }
 
 _lock = threading.Lock()

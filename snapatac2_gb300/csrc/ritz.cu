@@ -27,8 +27,8 @@
 //              moves their residuals by ~eps ‖T‖.  Two steps of a quadratic
 //              iteration spread over the GPU (0.26 ms for 288 vectors of
 //              length 336; a Cholesky-QR with its factor on one CTA took 7.0);
-//              vectors too far off for it (an inverse iteration that did not
-//              converge) still take the Cholesky-QR.
+//              vectors too far off for two steps (an inverse iteration that
+//              did not converge) still take the Cholesky-QR.
 //
 // Every sum runs in a fixed order, so results are reproducible run to run.
 #include <cooperative_groups.h>
@@ -549,8 +549,11 @@ __global__ void invit_kernel(int n, const double* __restrict__ d, const double* 
 }
 
 // E = Zt Ztᵀ - I over the nw rows of length n, both triangles; one warp per
-// entry of the lower one.  *wide counts the entries too large for the
-// iteration below: with every |E_ij| <= 1 / (4 nw), ‖E‖ <= 1/4.
+// entry of the lower one.  *wide counts the entries too large for the two
+// steps below: with every |E_ij| <= kOrthNear / nw, ‖E‖ <= kOrthNear, and two
+// steps of E -> 3/4 E² leave 0.42 kOrthNear⁴ = 4e-17.  Vectors of an inverse
+// iteration that converged are within it: eps / 1e-9 for the closest pairs.
+constexpr double kOrthNear = 1e-4;
 __global__ void gram_rows_kernel(int nw, int n, const double* __restrict__ Zt, double* __restrict__ E,
                                  int* __restrict__ wide) {
   const int lane = threadIdx.x & 31;
@@ -571,7 +574,7 @@ __global__ void gram_rows_kernel(int nw, int n, const double* __restrict__ Zt, d
     if (i == j) s -= 1.0;
     E[(size_t)i * nw + j] = s;
     E[(size_t)j * nw + i] = s;
-    if (wide && !(fabs(s) * (4.0 * nw) <= 1.0)) atomicAdd(wide, 1);
+    if (wide && !(fabs(s) * nw <= kOrthNear)) atomicAdd(wide, 1);
   }
 }
 
@@ -880,6 +883,27 @@ int ritz_values(int n, const double* A, int64_t lda, int p, int q, const RitzLay
   return SG_OK;
 }
 
+// The nw rows of Z (length n) to the closest orthonormal set, by two steps of
+// the iteration, or by Cholesky-QR where they are too far off.  Z2: as large
+// as Z; G: nw x nw.
+static int orth_rows(int nw, int n, double* Z, double* Z2, double* G, int* wide, cudaStream_t s) {
+  if (nw < 2) return SG_OK;
+  const int64_t pairs = (int64_t)nw * (nw + 1) / 2;
+  const dim3 grid((n + 127) / 128, (nw + kOrthRows - 1) / kOrthRows);
+  if (cudaMemsetAsync(wide, 0, sizeof(int), s) != cudaSuccess) return SG_ERR_CUDA;
+  gram_rows_kernel<<<grid_for(pairs * 32, 256), 256, 0, s>>>(nw, n, Z, G, wide);
+  SG_CHECK_LAUNCH();
+  orth_kernel<<<1, 1024, 0, s>>>(nw, n, G, Z, wide);
+  SG_CHECK_LAUNCH();
+  orth_step_kernel<<<grid, 128, 0, s>>>(nw, n, G, Z, Z2, wide);
+  SG_CHECK_LAUNCH();
+  gram_rows_kernel<<<grid_for(pairs * 32, 256), 256, 0, s>>>(nw, n, Z2, G, nullptr);
+  SG_CHECK_LAUNCH();
+  orth_step_kernel<<<grid, 128, 0, s>>>(nw, n, G, Z2, Z, wide);
+  SG_CHECK_LAUNCH();
+  return SG_OK;
+}
+
 // Eigenvectors of the nsel selected eigenvalues (sel: ascending indices into
 // L.lam, device; null = all *nw of them) into the first nsel rows of L.Zt.
 int ritz_vectors(int n, const RitzLayout& L, const int* sel, int nsel, cudaStream_t s) {
@@ -893,25 +917,8 @@ int ritz_vectors(int n, const RitzLayout& L, const int* sel, int nsel, cudaStrea
     backtr_kernel<<<nsel, kBackThreads, 0, s>>>(n, L.V, L.T, L.Zt);
     SG_CHECK_LAUNCH();
   }
-  if (nsel > 1) {
-    // two steps of the iteration through the inverse iteration's scratch and
-    // back; the second finds ‖E‖ <= 3/64 at worst and about 1e-14 as a rule
-    double* Z2 = L.lu;
-    const int64_t pairs = (int64_t)nsel * (nsel + 1) / 2;
-    const dim3 grid((n + 127) / 128, (nsel + kOrthRows - 1) / kOrthRows);
-    if (cudaMemsetAsync(L.wide, 0, sizeof(int), s) != cudaSuccess) return SG_ERR_CUDA;
-    gram_rows_kernel<<<grid_for(pairs * 32, 256), 256, 0, s>>>(nsel, n, L.Zt, L.G, L.wide);
-    SG_CHECK_LAUNCH();
-    orth_kernel<<<1, 1024, 0, s>>>(nsel, n, L.G, L.Zt, L.wide);
-    SG_CHECK_LAUNCH();
-    orth_step_kernel<<<grid, 128, 0, s>>>(nsel, n, L.G, L.Zt, Z2, L.wide);
-    SG_CHECK_LAUNCH();
-    gram_rows_kernel<<<grid_for(pairs * 32, 256), 256, 0, s>>>(nsel, n, Z2, L.G, nullptr);
-    SG_CHECK_LAUNCH();
-    orth_step_kernel<<<grid, 128, 0, s>>>(nsel, n, L.G, Z2, L.Zt, L.wide);
-    SG_CHECK_LAUNCH();
-  }
-  return SG_OK;
+  // two steps through the inverse iteration's scratch and back
+  return orth_rows(nsel, n, L.Zt, L.lu, L.G, L.wide, s);
 }
 
 }  // namespace sg
@@ -941,4 +948,17 @@ extern "C" int sg_sym_eig(int n, const double* A, int64_t lda, int p, int q, dou
       cudaMemcpyAsync(evecs, L.Zt, sizeof(double) * nw * (size_t)n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return SG_ERR_CUDA;
   return SG_OK;
+}
+
+extern "C" int64_t sg_orth_rows_work_bytes(int nw, int n) {
+  if (nw < 1 || n < nw || n > kRitzMaxN) return -1;
+  return 8 * ((int64_t)nw * n + (int64_t)nw * nw) + 8;
+}
+
+extern "C" int sg_orth_rows(int nw, int n, double* Z, void* work, int64_t work_bytes, void* stream) {
+  if (nw < 1 || n < nw || n > kRitzMaxN || !Z || !work || ((uintptr_t)work & 7u) != 0) return SG_ERR_ARG;
+  if (work_bytes < sg_orth_rows_work_bytes(nw, n)) return SG_ERR_CAP;
+  double* Z2 = static_cast<double*>(work);
+  double* G = Z2 + (int64_t)nw * n;
+  return orth_rows(nw, n, Z, Z2, G, reinterpret_cast<int*>(G + (int64_t)nw * nw), as_stream(stream));
 }
