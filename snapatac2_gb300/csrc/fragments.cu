@@ -25,8 +25,7 @@
 //             of processed groups, the minimum-fragment filter;
 //   order     kept groups by first appearance (sorted input) or by barcode
 //             bytes: by counting up to kRankGroups groups of up to 64 bytes,
-//             else by LSD radix
-//             (over length, then 8-byte big-endian words);
+//             else by LSD radix (over length, then 8-byte big-endian words);
 //   matrix    kept in-genome records keyed (cell, position, size), brought
 //             into order (see order_matrix) and decoded into CSR order.
 #include "common.cuh"
@@ -155,11 +154,12 @@ __global__ void __launch_bounds__(kThreads) line_fill_kernel(const uint8_t* __re
   __shared__ int wsum[2][kThreads / 32];
   int64_t base = before[c];  // newlines before this chunk
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool wide = ((uintptr_t)text & 15) == 0;  // p0 is a multiple of 16
   int turn = 0;
   for (int64_t r0 = b0; r0 < b1; r0 += kFillBytes * kThreads, turn ^= 1) {
     const int64_t p0 = r0 + kFillBytes * (int64_t)threadIdx.x;
     uint64_t m = 0;
-    if (p0 + kFillBytes <= b1) {
+    if (wide && p0 + kFillBytes <= b1) {
 #pragma unroll
       for (int v = 0; v < kFillBytes / 16; ++v)
         m |= (uint64_t)nl_bits(__ldg(reinterpret_cast<const uint4*>(text + p0) + v)) << (16 * v);
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kThreads) parse_kernel(const uint8_t* __restri
     const int64_t base = line_start[i0] & ~(int64_t)15;
     int64_t stop = line_start[il];
     if (stop > nbytes) stop = nbytes;
-    const bool staged = stop - base <= kStage;  // uniform
+    const bool staged = stop - base <= kStage && ((uintptr_t)text & 15) == 0;  // uniform; 16-byte loads
     __syncthreads();
     if (staged) {
       for (int64_t p = base + 16 * threadIdx.x; p < stop; p += 16 * kThreads) {
