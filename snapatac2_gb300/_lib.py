@@ -168,7 +168,7 @@ class LanczosInfo(ctypes.Structure):
 # benchmark): e.g. sg_block_cholqr = Gram partials + their sum and Cholesky +
 # R⁻¹ application.
 KERNELS_PER_CALL = {
-    "sg_tile_plan": 4, "sg_tile_bound": 1, "sg_tile_run": 5, "sg_tile_emit": 1, "sg_col_counts": 2, "sg_csr_select_cols": 5,
+    "sg_tile_plan": 4, "sg_tile_bound": 1, "sg_tile_run": 6, "sg_tile_emit": 1, "sg_col_counts": 2, "sg_csr_select_cols": 5,
     "sg_csr_transpose": 8, "sg_spectral_prepare": 7, "sg_spmm": 1, "sg_spmm_ex": 1, "sg_spmm_masked": 1, "sg_spmm_fx": 3, "sg_spmm_fx_counts": 3, "sg_counts_max": 1,
     "sg_spmm_staged": 1, "sg_spmm_dyn": 1, "sg_spmm_ds": 1, "sg_ds_split": 1, "sg_spmm_dyn_ordered": 1, "sg_row_order": 10, "sg_idf_from_counts": 3, "sg_csr_row_norms": 1, "sg_staged_table": 1, "sg_gather_ceiling": 1, "sg_block_proj": 2, "sg_block_update": 1, "sg_block_cholqr": 3, "sg_block_finish": 1,
     "sg_lanczos_hblock": 1, "sg_basis_rotate": 1, "sg_fill_random": 1, "sg_knn": 8, "sg_knn_noalloc": 8,
