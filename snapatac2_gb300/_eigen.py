@@ -130,10 +130,13 @@ class GramOperator:
             scale, dsh, yp = a.data_ptr(), dinv.data_ptr(), y.data_ptr()
             mask = self.row_mask.data_ptr() if self.row_mask is not None else None
         if variant >= FX:
-            if dtype_code == 1 and mask is None and (val is None or variant == FX_COUNTS and self.holds_counts(stream)):
+            if (dtype_code == 1 and mask is None and fx_pays(self.csr.nnz, block) and
+                    (val is None or variant == FX_COUNTS and self.holds_counts(stream))):
                 spmm_fx(rows, ptr, idx, cols, inp, out, scale, block, stream, dsh, yp, val)
                 return _lib.SG_OK
-            variant = 1
+            # one index chunk in flight for the short rows of the Xᵀ pass, two for
+            # the X pass: the fastest or within 10 % of it at 5,000 to 4e5 nonzeros
+            variant = which if dtype_code == 1 and mask is None else 1
         if variant >= DYN and dtype_code != 0:
             variant -= DYN  # the dynamic schedule exists for FP32 only: same gathers, static schedule
         if variant >= DYN:
@@ -206,6 +209,15 @@ FX = 300
 FX_COUNTS = 301
 
 
+def fx_pays(nnz: int, block: int) -> bool:
+    """Whether a fixed-point pass called from here is worth its three launches
+    and its scratch: 20 operator products of 1.7e6 values (nonzeros x columns)
+    take 866 us that way and 762 as FP64 additions, of 2e4 values 817 and 214,
+    of 3.3e6 values 845 and 1,002.  (sg_lanczos, which launches from C and has
+    its scratch, is not slower at any size.)"""
+    return nnz * block >= 3_000_000
+
+
 def spmm_fx(rows: int, ptr, idx, in_rows: int, inp, out, scale: int, block: int, stream: int, dshift=None,
             y=None, counts: int | None = None) -> None:
     """One FP64 SpMM of an implicit-ones CSR by exact fixed-point sums
@@ -228,11 +240,11 @@ def spmm_fx(rows: int, ptr, idx, in_rows: int, inp, out, scale: int, block: int,
 
 def spmm64(rows: int, ptr, idx, val, in_rows: int, inp, out, scale, block: int, stream: int) -> None:
     """out = scale ⊙ (X inp) in FP64: fixed-point sums when X holds ones
-    only, FP64 multiply-adds when it has values."""
-    if val is None:
+    only and enough of them, FP64 multiply-adds when it has values or few."""
+    if val is None and fx_pays(idx.numel(), block):
         spmm_fx(rows, ptr, idx, in_rows, inp, out, scale.data_ptr(), block, stream)
         return
-    _lib.check(_lib.load().sg_spmm(1, block, rows, ptr.data_ptr(), idx.data_ptr(), val.data_ptr(), inp.data_ptr(),
+    _lib.check(_lib.load().sg_spmm(1, block, rows, ptr.data_ptr(), idx.data_ptr(), _lib.ptr(val), inp.data_ptr(),
                                    out.data_ptr(), scale.data_ptr(), None, None, -1, stream), "sg_spmm (FP64)")
 
 _TUNED: dict = {}
