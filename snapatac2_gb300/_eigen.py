@@ -226,9 +226,14 @@ def spmm_fx(rows: int, ptr, idx, in_rows: int, inp, out, scale: int, block: int,
     device addresses."""
     L = _lib.load()
     nb = int(L.sg_spmm_fx_work_bytes(block, in_rows))
-    work = torch.empty(max(nb, 16), dtype=torch.uint8, device=inp.device)
-    if stream != torch.cuda.current_stream(inp.device).cuda_stream:  # freed on the current stream, used on another
-        work.record_stream(torch.cuda.ExternalStream(stream, device=inp.device))
+    # from the memory of the stream that uses it: a block of the current
+    # stream's may still be in use there, and nothing makes `stream` wait for it
+    if stream == torch.cuda.current_stream(inp.device).cuda_stream:
+        work = torch.empty(max(nb, 16), dtype=torch.uint8, device=inp.device)
+    else:
+        on = torch.cuda.ExternalStream(stream, device=inp.device) if stream else torch.cuda.default_stream(inp.device)
+        with torch.cuda.stream(on):
+            work = torch.empty(max(nb, 16), dtype=torch.uint8, device=inp.device)
     if counts is not None:
         _lib.check(L.sg_spmm_fx_counts(block, rows, ptr.data_ptr(), idx.data_ptr(), counts, in_rows, inp.data_ptr(),
                                        out.data_ptr(), scale, dshift, y, work.data_ptr(), nb, stream),
