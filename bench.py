@@ -155,7 +155,7 @@ class LaunchCounter:
 
             def wrap(*a, _fn=fn, _k=self.table[name]):
                 if self.active:
-                    self.count += _k
+                    self.count += _k(*a) if callable(_k) else _k
                 return _fn(*a)
             setattr(self.lib, name, wrap)
 

@@ -164,14 +164,26 @@ class LanczosInfo(ctypes.Structure):
                 ("seconds_restart", _F64), ("seconds_refine", _F64), ("spmm_ms_t", _F64), ("spmm_ms_x", _F64),
                 ("spmm_launches", _I64), ("kernel_launches", _I64)]
 
+def _cholqr_kernels(dtype, block, *_):
+    """Gram partials, their sum and Cholesky (blocks of 16 and 32: two
+    launches), R⁻¹ application."""
+    return 3 if block <= 8 else 4
+
+
+def _knn_kernels(X, n, d, *_):
+    """Eight; on ordered points (csrc/knn.cu, kOrderMin) also the codes, three
+    radix passes of five and the permutation, and up to 32 dimensions the
+    tensor-core tiles and their boxes."""
+    return 8 if n < 16385 else (27 if d <= 32 else 25)
+
+
 # Kernels launched by one call of each entry point (launch accounting of the
-# benchmark): e.g. sg_block_cholqr = Gram partials + their sum and Cholesky +
-# R⁻¹ application.
+# benchmark): a number, or a function of the call's arguments.
 KERNELS_PER_CALL = {
     "sg_tile_plan": 4, "sg_tile_bound": 1, "sg_tile_run": 6, "sg_tile_emit": 1, "sg_col_counts": 2, "sg_csr_select_cols": 5,
     "sg_csr_transpose": 8, "sg_spectral_prepare": 7, "sg_spmm": 1, "sg_spmm_ex": 1, "sg_spmm_masked": 1, "sg_spmm_fx": 3, "sg_spmm_fx_counts": 3, "sg_counts_max": 1,
-    "sg_spmm_staged": 1, "sg_spmm_dyn": 1, "sg_spmm_ds": 1, "sg_ds_split": 1, "sg_spmm_dyn_ordered": 1, "sg_row_order": 10, "sg_idf_from_counts": 3, "sg_csr_row_norms": 1, "sg_staged_table": 1, "sg_gather_ceiling": 1, "sg_block_proj": 2, "sg_block_update": 1, "sg_block_cholqr": 3, "sg_block_finish": 1,
-    "sg_lanczos_hblock": 1, "sg_basis_rotate": 1, "sg_fill_random": 1, "sg_knn": 8, "sg_knn_noalloc": 8,
+    "sg_spmm_staged": 1, "sg_spmm_dyn": 1, "sg_spmm_ds": 1, "sg_ds_split": 1, "sg_spmm_dyn_ordered": 1, "sg_row_order": 10, "sg_idf_from_counts": 3, "sg_csr_row_norms": 1, "sg_staged_table": 1, "sg_gather_ceiling": 1, "sg_block_proj": 2, "sg_block_update": 1, "sg_block_cholqr": _cholqr_kernels, "sg_block_finish": 1,
+    "sg_lanczos_hblock": 1, "sg_basis_rotate": 1, "sg_fill_random": 1, "sg_knn": _knn_kernels, "sg_knn_noalloc": 8,
     "sg_bblock_proj": 2, "sg_bblock_update": 1, "sg_bblock_cholqr": 4, "sg_blanczos_hblock": 1,
     "sg_bbasis_rotate": 1, "sg_bidf": 3, "sg_bmask": 1,
     "sg_adjoint_stage1": 1, "sg_adjoint_stage2": 1, "sg_adjoint_stage3": 1, "sg_adjoint_final": 1,
