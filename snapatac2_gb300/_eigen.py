@@ -270,9 +270,10 @@ def tune_spmm(op: "GramOperator", code: int, block: int, Z, Zs, T, W, stream: in
     >= 200 the dynamically scheduled gather kernel, 300 the fixed-point one).
 
     FP64 without values or masks, and with counts for values, is not timed:
-    the fixed-point kernel is the faster one at every size measured (Xᵀ pass
-    of 3.1e6 nonzeros, block 8: 38 us against 95; of 8.3e7, block 4: 0.34 ms
-    against 0.97; counts, 2.1e7 nonzeros, block 8: 191 us against 663).
+    the fixed-point kernel is the faster one in the solver at every size
+    measured (Xᵀ pass of 3.1e6 nonzeros, block 8: 38 us against 95; of 8.3e7,
+    block 4: 0.34 ms against 0.97; counts, 2.1e7 nonzeros, block 8: 213 us
+    against 663), and from fx_pays on from Python.
     """
     import os
     forced = os.environ.get("SNAPGB300_SPMM_VARIANT")

@@ -28,7 +28,8 @@
 // additions round at its size in one lane of eight only, and at 2^55 the two
 // errors are equal (0.6 sqrt(len) units).  In solves of 1,200 to 12,000 cells
 // with IDF weights no row goes that way; with weights spread as e^N(0,1) 0.3 %
-// of the rows of the X pass, as e^(3 N(0,1)) 8 %.  Looking costs 3 % of the Xᵀ
+// of the rows of the X pass, as e^(3 N(0,1)) 8 % (an embedding of 5,000 cells:
+// 21.5 ms, then 26.2; by FP64 additions alone 57).  Looking costs 3 % of the Xᵀ
 // pass (137 -> 141 us below), nothing in the X pass.
 //
 // Layout: CTAs of 8 warps own R consecutive rows, and each warp an equal slice
@@ -50,7 +51,7 @@
 // 4 columns 0.34 / 0.33 ms (0.97 / 0.74), 32 columns 0.99 / 1.17 ms (6.1 /
 // 5.9), where the 256-byte rows arrive at 22 / 18 TB/s.  (A warp per short row
 // and a CTA per long one: 167 / 159, 39 / 40, 390 / 430, 1,390 / 1,850.)  The
-// L1's lookups bind now (85-89 % of its peak throughput).
+// L1's lookups bind now (83-90 % of its peak throughput).
 //
 // Counts (COUNTS): a tile matrix holds whole numbers; an operand's integer
 // times a count below 2^16 is two wide integer multiplications, and with a
@@ -79,7 +80,8 @@ constexpr int kFxMaxRows = kFxWarps * (64 / B);  // rows per CTA at most
 constexpr int kHeadBytes = 256;    // per-column maxima in front of the integers
 constexpr unsigned kNonFinite = 0x7ff00000u;
 constexpr unsigned kVouch = 55;    // exponent of the magnitudes that vouch for a sum
-constexpr int kLook = 4;           // COUNTS: of a row's gathers, those looked at for such (all in the last 32 entries)
+constexpr int kLook = 4;           // COUNTS: every fourth gather of 32 entries (4 columns: every second) is looked at for
+                                   // such, and all of a row's last 32 entries
 
 // scale exponent of a column whose largest |x| has this high word: |x| 2^s < 2^63
 __device__ __forceinline__ int fx_shift(unsigned maxhi) {

@@ -171,9 +171,9 @@ __device__ __forceinline__ bool row_ok(int64_t K, int64_t kbase, int64_t key_cap
 // The radix sort it replaces moved every key through shared memory in three
 // passes of six barriers per 512 keys, at one CTA per SM (200 KB), and
 // through L2 for the third of the cells above 24,576 keys: 4.87 ms for 5,000
-// cells and 6.1e7 fragments, 0.72 ms here (1.0 TB/s of fragments in, at four
+// cells and 6.1e7 fragments, 0.7 ms here (1.0 TB/s of fragments in, at four
 // CTAs of 64 registers per SM; instruction issue and barriers bind).  The call
-// went from 6.07 to 1.07 ms with the pass that planned it left out (0.53 ms)
+// went from 6.07 to 1.06 ms with the pass that planned it left out (0.53 ms)
 // and one read back instead of five.  Cells that break
 // the assumptions (unsorted or zero-length fragments, or a chunk that covers
 // more tiles than there are slots) are left to sort_kernel: cell_nnz = -1.
